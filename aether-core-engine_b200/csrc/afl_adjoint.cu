@@ -118,6 +118,9 @@ struct afl_adjoint {
   afl::PersistentState ps{};
   afl::ResidentPlan res{};  // on-chip CG tiles, when the grid fits
   bool resident = false;
+  afl::BrickPlan brick{};   // ... and its bricks, when it fits those
+  bool brick_ok = false;
+  void *brick_scratch = nullptr;
   std::vector<std::array<double *, 6>> ckpt;
   std::vector<Rec> rec;
   // adjoint work arrays
@@ -164,13 +167,19 @@ afl_status copy(afl_adjoint *a, double *dst, const double *src) {
   return AFL_OK;
 }
 
-// The FP64 CG of afl_solve_cg (warm start from x): the on-chip resident
-// kernel when the grid fits, else the streaming one.
+// The FP64 CG of afl_solve_cg (warm start from x): the brick-resident kernel
+// when the grid fits, then the column-resident one, else the streaming one.
 afl_status solve(afl_adjoint *a, double *x, const double *rhs, long *iters) {
   int used;
+  const int *abort_word = a->ps.abort_flag;
   if (a->params.solver_kind == AFL_POISSON_RBSOR) {
     afl::SorArgs sa{a->g, x, rhs, a->params.solver_iters, a->params.sor_omega, a->rep};
     used = afl::launch_rbsor_f64(sa, a->ps, a->stream);
+  } else if (a->resident && a->brick_ok) {
+    const afl::BrickSolve ba{a->g, x, rhs, a->brick_scratch, a->params.solver_iters,
+                             a->params.cg_rel_tol, a->rep, a->ps.timeout_ns};
+    used = afl::launch_cg_brick(ba, a->brick, a->stream);
+    abort_word = static_cast<const int *>(a->brick_scratch);
   } else if (a->resident) {
     afl::ResidentCgArgs ra{};
     ra.g = a->g;
@@ -191,7 +200,7 @@ afl_status solve(afl_adjoint *a, double *x, const double *rhs, long *iters) {
   ADJ_CUDA(cudaMemcpyAsync(&r, a->rep, sizeof r, cudaMemcpyDeviceToHost, a->stream));
   ADJ_CUDA(cudaStreamSynchronize(a->stream));
   int abort_flag = 0;
-  ADJ_CUDA(cudaMemcpy(&abort_flag, a->ps.abort_flag, sizeof abort_flag, cudaMemcpyDeviceToHost));
+  ADJ_CUDA(cudaMemcpy(&abort_flag, abort_word, sizeof abort_flag, cudaMemcpyDeviceToHost));
   if (abort_flag) return fail(AFL_ERR_TIMEOUT, "the CG kernel gave up at a grid barrier");
   if (r.status != 0) return fail(AFL_ERR_NONFINITE, "non-finite residual in a CG solve");
   *iters += r.iterations;
@@ -423,13 +432,28 @@ afl_status afl_adjoint_create(size_t nx, size_t ny, size_t nz, const afl_params 
   for (double **x : singles)
     if (st == AFL_OK) st = dalloc(a, x);
   for (int f = 0; f < 4 && st == AFL_OK; ++f) st = dalloc(a, &a->curl[f]);
-  // one block: the resident FP64 CG reads cg[0..3] as four consecutive arrays
+  // The Poisson kernel follows params->poisson_kernel as afl_create's does:
+  // AUTO takes an on-chip resident CG when the grid fits, STREAMING never,
+  // RESIDENT always (an error when the grid does not fit).
+  const int maxb = afl::persistent_blocks_cg_f64();
+  const bool fits = afl::plan_resident(a->g, true, &a->res) &&
+                    a->res.tiles_x * a->res.tiles_y <= maxb;
+  if (params->poisson_kernel == AFL_POISSON_KERNEL_RESIDENT && !fits)
+    return bail(fail(AFL_ERR_INVALID_ARGUMENT,
+                     "the grid does not fit the resident CG kernel"));
+  a->resident = fits && params->poisson_kernel != AFL_POISSON_KERNEL_STREAMING;
+  a->brick_ok = a->resident && afl::plan_brick(a->g, &a->brick);
+  // one block: the resident FP64 CG reads cg[0..3] as four consecutive arrays,
+  // the brick-resident one keeps its slots and inboxes there
   if (st == AFL_OK) {
     void *blk = nullptr;
-    if (cudaMalloc(&blk, 4 * nbytes(a)) != cudaSuccess) {
+    size_t bytes = 4 * nbytes(a);
+    if (a->brick_ok) bytes = std::max(bytes, afl::brick_scratch_bytes(a->brick));
+    if (cudaMalloc(&blk, bytes) != cudaSuccess) {
       st = fail(AFL_ERR_OUT_OF_MEMORY, "CG vectors");
     } else {
       a->allocs.push_back(blk);
+      a->brick_scratch = blk;
       for (int f = 0; f < 4; ++f) a->cg[f] = static_cast<double *>(blk) + f * static_cast<size_t>(a->g.n);
     }
   }
@@ -450,7 +474,6 @@ afl_status afl_adjoint_create(size_t nx, size_t ny, size_t nz, const afl_params 
     return bail(fail(AFL_ERR_OUT_OF_MEMORY, "report"));
   a->allocs.push_back(v);
   a->rep = static_cast<afl::SolveReport *>(v);
-  const int maxb = afl::persistent_blocks_cg_f64();
   if (cudaMalloc(&v, sizeof(unsigned int) * 4) != cudaSuccess)
     return bail(fail(AFL_ERR_OUT_OF_MEMORY, "barrier"));
   a->allocs.push_back(v);
@@ -465,15 +488,6 @@ afl_status afl_adjoint_create(size_t nx, size_t ny, size_t nz, const afl_params 
   a->ps.partials = static_cast<double *>(v);
   a->ps.max_blocks = maxb;
   a->ps.timeout_ns = 5000000000ull;
-  // The Poisson kernel follows params->poisson_kernel as afl_create's does:
-  // AUTO takes the on-chip resident CG when the grid fits, STREAMING never,
-  // RESIDENT always (an error when the grid does not fit).
-  const bool fits = afl::plan_resident(a->g, true, &a->res) &&
-                    a->res.tiles_x * a->res.tiles_y <= maxb;
-  if (params->poisson_kernel == AFL_POISSON_KERNEL_RESIDENT && !fits)
-    return bail(fail(AFL_ERR_INVALID_ARGUMENT,
-                     "the grid does not fit the resident CG kernel"));
-  a->resident = fits && params->poisson_kernel != AFL_POISSON_KERNEL_STREAMING;
   // one segment of recorded steps
   a->rec.resize(static_cast<size_t>(a->k));
   for (Rec &R : a->rec) {

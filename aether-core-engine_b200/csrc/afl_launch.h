@@ -198,6 +198,35 @@ size_t resident_smem_bytes(const Dims &g, int ty, int cpt, bool f64);
 int launch_cg_resident(const ResidentCgArgs &a, const ResidentPlan &plan, bool f64,
                        const PersistentState &ps, cudaStream_t st);
 
+// Brick-resident FP64 CG (afl_poisson_brick.cu): one 512-thread CTA per SM owns
+// a bx x (512/bx) x cz brick.
+constexpr int kBrickMaxPlanes = 32;
+constexpr size_t kBrickHeader = 64;  // scratch: abort flag, then the sums' slots, the inboxes
+struct BrickPlan {
+  int bx;             // brick width in x (the brick has 512/bx rows)
+  int nbx, nby, nbz;  // bricks per axis
+  int cz;             // planes per brick
+  size_t smem_bytes;  // dynamic shared memory per CTA
+  size_t inbox_bytes;
+  int ctas() const { return nbx * nby * nbz; }
+};
+struct BrickSolve {
+  Dims g;
+  double *p;        // pressure (warm start in, solution out)
+  const double *b;  // right-hand side
+  void *scratch;    // brick_scratch_bytes(plan) bytes, 16-byte aligned; its first word is
+                    // the abort flag after the launch
+  int max_iters;
+  double rel_tol;
+  SolveReport *report;
+  unsigned long long timeout_ns;
+};
+// False when the grid needs more bricks than SMs.
+bool plan_brick(const Dims &g, BrickPlan *plan);
+size_t brick_scratch_bytes(const BrickPlan &plan);
+// Returns the CTAs launched, or minus a cudaError_t.
+int launch_cg_brick(const BrickSolve &s, const BrickPlan &plan, cudaStream_t st);
+
 // The two orbiting jets of inject_cyberpunk_sources (src/fluid.rs:533-571) at
 // time_sec: centre and velocity of each jet, its cell box clamped as the
 // reference clamps it, the squared radius in cells and the pulse.

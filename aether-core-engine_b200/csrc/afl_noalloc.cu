@@ -5,12 +5,13 @@
 // the device and takes driver locks), and hosts whose device memory is owned
 // entirely by their own pool or arena (a game engine's or a renderer's
 // budgeted heap), where a hidden allocation by a library breaks the budget.
-// For them afl_solve_cg_noalloc runs the streaming persistent FP64 CG kernel
-// (the kernel afl_solve_cg runs with AFL_POISSON_KERNEL_STREAMING; its AUTO
-// choice may run the on-chip resident kernel instead, whose sums are ordered
-// differently) on device buffers the caller already owns, and takes the
-// solver's working memory from one fixed array compiled into this library
-// instead of allocating it.  The call synchronises its stream before it
+// For them afl_solve_cg_noalloc runs the brick-resident FP64 CG kernel when the
+// grid fits it (the kernel afl_solve_cg's AUTO choice runs), else the streaming
+// persistent one (AFL_POISSON_KERNEL_STREAMING), on device buffers the caller
+// already owns, and takes the solver's working memory from one fixed array
+// compiled into this library instead of allocating it.  At these sizes an
+// iteration is all latency: the streaming kernel's two barriers cost 14 us on
+// 40 x 36 x 30, the brick kernel's one sum 3 us.  The call synchronises its stream before it
 // returns, to read the solve's report.
 //
 // The array below is that working memory.  Every GPU that loads the library
@@ -103,19 +104,10 @@ extern "C" afl_status afl_solve_cg_noalloc(const double *d_rhs, double *d_pressu
   if (blocks > kMaxPartialBlocks)
     return fail(AFL_ERR_CUDA, "this GPU needs more persistent CTAs than the scratch holds");
 
-  // Carve the array: barrier words and report, partials, then r, d0, d1, q.
-  auto *words = reinterpret_cast<unsigned int *>(base);
-  auto *report = reinterpret_cast<afl::SolveReport *>(base + 64);
-  auto *partials = reinterpret_cast<double *>(base + kHeaderBytes);
-  auto *vec = reinterpret_cast<double *>(base + kHeaderBytes + kPartialBytes);
+  // The brick kernel's scratch (its sums' slots and inboxes) takes the vectors'
+  // place behind the header.
+  afl::BrickPlan plan{};
   const size_t n = nx * ny * nz;
-
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // Zero what a call must not inherit from the previous one: the barrier
-  // words and the report (the partials and vectors are written before read).
-  e = cudaMemsetAsync(base, 0, kHeaderBytes, s);
-  if (e != cudaSuccess) return fail(AFL_ERR_CUDA, cudaGetErrorString(e));
-
   afl::Dims g{};
   g.nx = static_cast<int>(nx);
   g.ny = static_cast<int>(ny);
@@ -123,6 +115,20 @@ extern "C" afl_status afl_solve_cg_noalloc(const double *d_rhs, double *d_pressu
   g.nxy = static_cast<int>(nx * ny);
   g.n = static_cast<int>(n);
   g.h = 1.0 / static_cast<double>(nx > ny ? (nx > nz ? nx : nz) : (ny > nz ? ny : nz));
+  const bool brick = afl::plan_brick(g, &plan) &&
+                     afl::brick_scratch_bytes(plan) <= kNoAllocBytes - kHeaderBytes;
+
+  // Carve the array: barrier words and report, partials, then r, d0, d1, q.
+  auto *words = reinterpret_cast<unsigned int *>(base);
+  auto *report = reinterpret_cast<afl::SolveReport *>(base + 64);
+  auto *partials = reinterpret_cast<double *>(base + kHeaderBytes);
+  auto *vec = reinterpret_cast<double *>(base + kHeaderBytes + kPartialBytes);
+
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // Zero what a call must not inherit from the previous one: the barrier
+  // words and the report (the partials and vectors are written before read).
+  e = cudaMemsetAsync(base, 0, kHeaderBytes, s);
+  if (e != cudaSuccess) return fail(AFL_ERR_CUDA, cudaGetErrorString(e));
 
   afl::PersistentState ps{};
   ps.count = words;
@@ -132,9 +138,18 @@ extern "C" afl_status afl_solve_cg_noalloc(const double *d_rhs, double *d_pressu
   ps.max_blocks = kMaxPartialBlocks;
   ps.timeout_ns = 5000000000ull;
 
-  afl::CgArgs a{g, d_pressure, d_rhs, vec, vec + n, vec + 2 * n, vec + 3 * n, max_iters,
-                rel_tol, report};
-  const int used = afl::launch_cg_f64(a, ps, s);
+  int used;
+  const void *abort_word = words + 2;
+  if (brick) {
+    abort_word = base + kHeaderBytes;
+    const afl::BrickSolve a{g, d_pressure, d_rhs, base + kHeaderBytes, max_iters, rel_tol, report,
+                            ps.timeout_ns};
+    used = afl::launch_cg_brick(a, plan, s);
+  } else {
+    const afl::CgArgs a{g, d_pressure, d_rhs, vec, vec + n, vec + 2 * n, vec + 3 * n, max_iters,
+                        rel_tol, report};
+    used = afl::launch_cg_f64(a, ps, s);
+  }
   if (used <= 0) {
     cudaGetLastError();
     return fail(AFL_ERR_CUDA, "cooperative launch of the CG kernel failed");
@@ -144,7 +159,7 @@ extern "C" afl_status afl_solve_cg_noalloc(const double *d_rhs, double *d_pressu
   int abort_flag = 0;
   e = cudaMemcpyAsync(&rep, report, sizeof rep, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&abort_flag, words + 2, sizeof abort_flag, cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(&abort_flag, abort_word, sizeof abort_flag, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(AFL_ERR_CUDA, cudaGetErrorString(e));
   if (abort_flag != 0)

@@ -126,6 +126,9 @@ struct afl_solver {
   afl::PersistentState ps{};
   bool resident_ok = false;       // the grid fits the on-chip resident CG
   afl::ResidentPlan resident{};
+  bool brick_ok = false;          // FP64: ... and the brick-resident CG too
+  afl::BrickPlan brick{};
+  void *brick_scratch = nullptr;  // the block of cg[]
   double *amp = nullptr;          // sphere amplitude map (optional)
   double *stage = nullptr;        // f64 staging for the mixed form's transfers
   double *sample_buf = nullptr;   // 4 doubles per point
@@ -341,13 +344,19 @@ afl_status stage_solve(afl_solver *s, int kind, int iters, afl::SolveReport *rep
   const Dims &g = s->g;
   StageTimer timer(s, AFL_STAGE_POISSON, 2);
   int blocks = 0;
+  const int *abort_flag = s->ps.abort_flag;
   const bool want_resident = kind == AFL_POISSON_CG &&
                              s->params.poisson_kernel != AFL_POISSON_KERNEL_STREAMING;
   if (kind == AFL_POISSON_CG && s->params.poisson_kernel == AFL_POISSON_KERNEL_RESIDENT &&
       !s->resident_ok)
     return set_error(AFL_ERR_INVALID_ARGUMENT,
                      "the %dx%dx%d grid does not fit the resident CG kernel", g.nx, g.ny, g.nz);
-  if (want_resident && s->resident_ok) {
+  if (want_resident && s->brick_ok) {
+    const afl::BrickSolve a{g, s->p, s->b, s->brick_scratch, iters, s->params.cg_rel_tol, rep,
+                            s->ps.timeout_ns};
+    blocks = afl::launch_cg_brick(a, s->brick, s->stream);
+    abort_flag = static_cast<const int *>(s->brick_scratch);
+  } else if (want_resident && s->resident_ok) {
     const bool f64 = s->precision == AFL_PRECISION_FP64;
     afl::ResidentCgArgs a{};
     a.g = g;
@@ -420,7 +429,7 @@ afl_status stage_solve(afl_solver *s, int kind, int iters, afl::SolveReport *rep
                      cudaGetErrorString(static_cast<cudaError_t>(-blocks)));
   }
   AFL_TRY(launch_check());
-  k_fold_status<<<1, 32, 0, s->stream>>>(s->ps.abort_flag, rep, s->sticky);
+  k_fold_status<<<1, 32, 0, s->stream>>>(abort_flag, rep, s->sticky);
   return launch_check();
 }
 
@@ -668,9 +677,16 @@ afl_status afl_create(size_t nx, size_t ny, size_t nz, const afl_params *params,
   if (st == AFL_OK) st = alloc_as(s, &s->p, n * sizeof(double));
   if (st == AFL_OK) st = alloc_as(s, &s->b, n * sizeof(double));
   const int ncg = s->precision == AFL_PRECISION_FP64 ? 4 : 5;
-  // one block: the resident FP64 CG reads cg[0..3] as four consecutive arrays
+  // one block: the resident FP64 CG reads cg[0..3] as four consecutive arrays,
+  // the brick-resident one keeps its slots and inboxes there
+  s->resident_ok = afl::plan_resident(s->g, s->precision == AFL_PRECISION_FP64, &s->resident);
+  s->brick_ok = s->resident_ok && s->precision == AFL_PRECISION_FP64 &&
+                afl::plan_brick(s->g, &s->brick);
+  size_t cg_bytes = fb * static_cast<size_t>(ncg);
+  if (s->brick_ok) cg_bytes = std::max(cg_bytes, afl::brick_scratch_bytes(s->brick));
   void *cg_block = nullptr;
-  if (st == AFL_OK) st = dev_alloc(s, &cg_block, fb * static_cast<size_t>(ncg));
+  if (st == AFL_OK) st = dev_alloc(s, &cg_block, cg_bytes);
+  s->brick_scratch = cg_block;
   for (int f = 0; f < ncg && st == AFL_OK; ++f)
     s->cg[f] = static_cast<unsigned char *>(cg_block) + fb * static_cast<size_t>(f);
   if (st == AFL_OK && s->precision == AFL_PRECISION_MIXED)
@@ -686,7 +702,6 @@ afl_status afl_create(size_t nx, size_t ny, size_t nz, const afl_params *params,
                       std::max(afl::persistent_blocks_cg_mixed(),
                                afl::persistent_blocks_sor_mixed()));
   s->ps.max_blocks = maxb;
-  s->resident_ok = afl::plan_resident(s->g, s->precision == AFL_PRECISION_FP64, &s->resident);
   s->ps.timeout_ns = 5000000000ull;  // 5 s per barrier wait
   if (const char *env = std::getenv("AFL_BARRIER_TIMEOUT_NS")) s->ps.timeout_ns = std::strtoull(env, nullptr, 10);
   unsigned int *bar = nullptr;

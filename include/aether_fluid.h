@@ -73,9 +73,11 @@ typedef enum afl_precision {
   AFL_PRECISION_MIXED = 1
 } afl_precision;
 
-/* Poisson kernel choice.  CG, AUTO: the on-chip resident kernel when the grid
- * fits (tiles <= SMs, tile + halo in shared memory), else the streaming
- * kernel; the two differ only in the summation order of the inner products.
+/* Poisson kernel choice.  CG, AUTO: an on-chip resident kernel when the grid
+ * fits (tiles <= SMs, tile + halo in shared memory; FP64 runs in bricks where
+ * the grid also splits into no more 512-column bricks than SMs, else in column
+ * tiles), else the streaming kernel; they differ only in the summation order of
+ * the inner products and in the rounding of fused updates.
  * RB-SOR, AUTO: the resident kernel for the mixed form when the grid fits,
  * else the streaming sweep; RESIDENT selects the resident sweep for FP64 too
  * (same result bit for bit, since a colour reads only the other colour). */
@@ -245,10 +247,11 @@ afl_status afl_set_stage_timing(afl_solver *s, int enable);
  * number of timed calls per stage (arrays of AFL_STAGE_COUNT; either may be
  * NULL). */
 afl_status afl_get_stage_timing(afl_solver *s, double *ms, int64_t *calls);
-/* The CG kernel plan chosen for this grid: out[0] = 1 when the on-chip
- * resident kernel fits (else the streaming kernel runs), out[1] = tile height
- * in y (tiles are 16 wide in x and span all z), out[2] = z cells per thread,
- * out[3] = CTAs (one per SM). */
+/* The column-tile plan of this grid, which decides whether a CG solve is
+ * resident: out[0] = 1 when it fits on chip (else the streaming kernel runs),
+ * out[1] = tile height in y (tiles are 16 wide in x and span all z), out[2] = z
+ * cells per thread, out[3] = CTAs (one per SM).  FP64 solves of a resident grid
+ * run in bricks where those fit too. */
 afl_status afl_get_poisson_plan(const afl_solver *s, int32_t out[4]);
 /* Kernels this handle has launched since creation. */
 afl_status afl_get_launch_count(const afl_solver *s, uint64_t *count);
@@ -387,8 +390,8 @@ afl_status afl_medium_sample_interaction(afl_medium *m, const afl_ray *rays, siz
  * No counterpart in the reference.  For callers that may not allocate device
  * memory -- real-time/render threads that must not block on the driver's
  * allocator, hosts whose device memory is one budgeted pool -- this runs the
- * streaming FP64 CG kernel (the one afl_solve_cg runs with
- * AFL_POISSON_KERNEL_STREAMING; same stopping rules, warm start from
+ * brick-resident FP64 CG kernel when the grid fits it, else the streaming one
+ * (the kernels afl_solve_cg runs; same stopping rules, warm start from
  * *d_pressure) on device buffers the caller owns: d_rhs (read) and d_pressure
  * (read and written), nx*ny*nz doubles each, x fastest.  Its working memory is
  * a fixed array inside the library (about 8.1 MiB, held on every GPU that

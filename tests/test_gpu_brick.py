@@ -1,0 +1,81 @@
+"""The brick-resident FP64 CG at the sizes where its bricks, faces and padding
+planes can go wrong, against the streaming kernel on the same system.  The two
+differ in the order of the sums and in the rounding of the fused updates, so 30
+iterations agree to 1e-10 of the pressure's norm (the bound the other resident
+kernels are held to)."""
+import numpy as np
+import pytest
+
+from helpers import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (6, 6, 6),       # one plane per brick, one column tile
+    (31, 7, 9), (33, 17, 300),   # one lane past a brick; 3 planes, 100 bricks in z
+    (32, 16, 592),   # 4 planes per brick, every SM
+    (20, 30, 40), (16, 40, 700),  # bricks 16 wide
+    (64, 64, 75), (64, 64, 128),  # 5 planes (a padded chunk), 8 planes
+    (96, 96, 97), (96, 96, 144),  # 13 and 16 planes
+    (128, 128, 125), (127, 113, 128),  # 32 planes, ragged in every axis
+    (200, 160, 20), (50, 330, 30),
+]
+
+
+def system(shape, seed, walls):
+    nx, ny, nz = shape
+    rng = np.random.default_rng(seed)
+    b = rng.standard_normal((nz, ny, nx)) * 0.01
+    inner = b[1:-1, 1:-1, 1:-1]
+    inner -= inner.mean()
+    if not walls:
+        full = np.zeros_like(b)
+        full[1:-1, 1:-1, 1:-1] = inner
+        b = full
+    return b.ravel(), rng.standard_normal(nx * ny * nz) * 0.01
+
+
+def solve(af, shape, kernel, b, p0, iters, rel_tol=0.0):
+    s = af.FluidSolver3D(*shape, poisson_kernel=kernel, cg_rel_tol=rel_tol)
+    s.set_field("divergence", b)
+    s.set_field("pressure", p0)
+    info = s.solve_poisson_conjugate_gradient(iters)
+    p = s.get_field("pressure")
+    s.close()
+    return p, info
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
+def test_brick_matches_streaming(af, shape):
+    b, p0 = system(shape, 5, False)
+    ref, ri = solve(af, shape, 1, b, p0, 30)
+    got, gi = solve(af, shape, 0, b, p0, 30)
+    assert gi.iterations == ri.iterations
+    assert rel_l2(got, ref) <= 1e-10
+    assert abs(gi.final_residual - ri.final_residual) <= 1e-9 * ri.rhs_norm
+
+
+@pytest.mark.parametrize("shape", [(31, 7, 9), (64, 64, 75), (50, 330, 30)])
+def test_brick_wall_cells_of_the_right_hand_side(af, shape):
+    """A caller's right-hand side may be non-zero on the walls, where the
+    operator's rows are zero: that part of the residual never shrinks and the
+    iteration soon diverges, so the first three iterations are compared."""
+    b, p0 = system(shape, 5, True)
+    ref, ri = solve(af, shape, 1, b, p0, 3)
+    got, gi = solve(af, shape, 0, b, p0, 3)
+    assert gi.iterations == ri.iterations == 3
+    assert rel_l2(got, ref) <= 1e-10
+
+
+def test_brick_stops_where_streaming_stops(af):
+    """Iteration budgets 0 and 1, a met tolerance, a zero right-hand side."""
+    shape = (40, 20, 18)
+    b, p0 = system(shape, 6, False)
+    for iters, tol in ((0, 0.0), (1, 0.0), (500, 1e-8)):
+        ref, ri = solve(af, shape, 1, b, p0, iters, tol)
+        got, gi = solve(af, shape, 0, b, p0, iters, tol)
+        assert abs(gi.iterations - ri.iterations) <= (1 if tol else 0)
+        assert gi.converged == ri.converged and rel_l2(got, ref) <= 1e-8
+    z = np.zeros_like(b)
+    got, gi = solve(af, shape, 0, z, z, 50)
+    assert gi.converged and gi.iterations == 0 and not got.any()
