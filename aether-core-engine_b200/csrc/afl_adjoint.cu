@@ -172,7 +172,12 @@ afl_status copy(afl_adjoint *a, double *dst, const double *src) {
 afl_status solve(afl_adjoint *a, double *x, const double *rhs, long *iters) {
   int used;
   const int *abort_word = a->ps.abort_flag;
-  if (a->params.solver_kind == AFL_POISSON_RBSOR) {
+  if (a->params.solver_kind == AFL_POISSON_RBSOR && a->brick_ok) {
+    const afl::BrickSor sa{a->g, x, rhs, a->brick_scratch, a->params.solver_iters,
+                           a->params.sor_omega, a->rep, a->ps.timeout_ns};
+    used = afl::launch_sor_brick(sa, a->brick, true, a->stream);
+    abort_word = static_cast<const int *>(a->brick_scratch);
+  } else if (a->params.solver_kind == AFL_POISSON_RBSOR) {
     afl::SorArgs sa{a->g, x, rhs, a->params.solver_iters, a->params.sor_omega, a->rep};
     used = afl::launch_rbsor_f64(sa, a->ps, a->stream);
   } else if (a->resident && a->brick_ok) {

@@ -36,18 +36,6 @@ __device__ __forceinline__ void st_packet(Packet *p, double v, unsigned tag) {
                : "memory");
 }
 
-// The same under a predicate (a predicated store, not a branch).
-__device__ __forceinline__ void st_packet_if(bool on, Packet *p, double v, unsigned tag) {
-  unsigned long long a, b;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "r"(__double2loint(v)), "r"(tag));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "r"(__double2hiint(v)), "r"(tag));
-  asm volatile(
-      "{\n.reg .pred on;\nsetp.ne.s32 on, %3, 0;\n"
-      "@on st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};\n}" ::"l"(p),
-      "l"(a), "l"(b), "r"(static_cast<int>(on))
-      : "memory");
-}
-
 // A packet on the way in; loading and checking are apart, so that several loads
 // are in flight at once (a packet that is not wanted reads as a tagged 0).
 struct RawPacket {
@@ -68,6 +56,44 @@ struct RawPacket {
     return __hiloint2double(static_cast<int>(b & 0xffffffffull),
                             static_cast<int>(a & 0xffffffffull));
   }
+};
+
+// The f32 form: one word.
+__device__ __forceinline__ void st_packet(unsigned long long *p, float v, unsigned tag) {
+  unsigned long long a;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "r"(__float_as_uint(v)), "r"(tag));
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(a) : "memory");
+}
+struct RawWord {
+  unsigned long long a;
+  __device__ __forceinline__ void ld(bool on, const unsigned long long *p, unsigned tag) {
+    a = static_cast<unsigned long long>(tag) << 32;
+    asm volatile(
+        "{\n.reg .pred on;\nsetp.ne.s32 on, %2, 0;\n"
+        "@on ld.relaxed.gpu.global.u64 %0, [%1];\n}"
+        : "+l"(a)
+        : "l"(p), "r"(static_cast<int>(on))
+        : "memory");
+  }
+  __device__ __forceinline__ bool has(unsigned tag) const {
+    return static_cast<unsigned>(a >> 32) == tag;
+  }
+  __device__ __forceinline__ float value() const {
+    return __uint_as_float(static_cast<unsigned>(a & 0xffffffffull));
+  }
+};
+// The packet of a value type: its word(s) in memory, and one on the way in.
+template <typename T>
+struct PacketOf;
+template <>
+struct PacketOf<double> {
+  using Mem = Packet;
+  using Raw = RawPacket;
+};
+template <>
+struct PacketOf<float> {
+  using Mem = unsigned long long;
+  using Raw = RawWord;
 };
 
 // Bookkeeping of a bounded wait: call once per failed poll; false = give up
@@ -235,6 +261,7 @@ template <typename S>
 struct BrickFaces {
   int xstage;         // this column's staged row (-1: not on an x face)
   int xdst;           // where the thread's first staged value goes; kSide packets per plane
+  int xcol;           // where plane 0 of an x-face column goes when it is sent directly
   int ydst;           // plane 0 of the column; kSide packets further per plane
   int zlo_dst, zhi_dst;
   int own;            // this CTA's inbox
@@ -258,7 +285,10 @@ struct BrickFaces {
       xdst = xs < S::BY ? (cl.bx > 0 ? box(-1, 0, 0) + S::BY + xs + m0 : -1)
                         : (cl.bx + 1 < nbx ? box(1, 0, 0) + xs - S::BY + m0 : -1);
     }
+    xcol = -1;
     if (cl.in_ij) {
+      if (ii == 0 && cl.bx > 0) xcol = box(-1, 0, 0) + S::BY + jj;
+      if (ii == S::BX - 1 && cl.bx + 1 < nbx) xcol = box(1, 0, 0) + jj;
       if (jj == 0 && cl.by > 0) ydst = box(0, -1, 0) + 2 * S::BY + S::BX + ii;
       if (jj == S::BY - 1 && cl.by + 1 < nby) ydst = box(0, 1, 0) + 2 * S::BY + ii;
       if (cl.bz > 0) zlo_dst = box(0, 0, -1) + zface + kBT + t;

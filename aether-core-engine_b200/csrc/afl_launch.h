@@ -224,6 +224,19 @@ struct BrickSolve {
 // False when the grid needs more bricks than SMs.
 bool plan_brick(const Dims &g, BrickPlan *plan);
 size_t brick_scratch_bytes(const BrickPlan &plan);
+// Red-black SOR on the same bricks (afl_sor_brick.cu): the FP64 pressure, or
+// the mixed form's f32 correction.  scratch: as for the CG.
+struct BrickSor {
+  Dims g;
+  double *p;
+  const double *b;
+  void *scratch;
+  int sweeps;
+  double omega;
+  SolveReport *report;
+  unsigned long long timeout_ns;
+};
+int launch_sor_brick(const BrickSor &s, const BrickPlan &plan, bool f64, cudaStream_t st);
 // Returns the CTAs launched, or minus a cudaError_t.
 int launch_cg_brick(const BrickSolve &s, const BrickPlan &plan, cudaStream_t st);
 

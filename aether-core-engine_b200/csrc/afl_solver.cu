@@ -126,7 +126,7 @@ struct afl_solver {
   afl::PersistentState ps{};
   bool resident_ok = false;       // the grid fits the on-chip resident CG
   afl::ResidentPlan resident{};
-  bool brick_ok = false;          // FP64: ... and the brick-resident CG too
+  bool brick_ok = false;          // ... and the brick-resident kernels
   afl::BrickPlan brick{};
   void *brick_scratch = nullptr;  // the block of cg[]
   double *amp = nullptr;          // sphere amplitude map (optional)
@@ -351,7 +351,7 @@ afl_status stage_solve(afl_solver *s, int kind, int iters, afl::SolveReport *rep
       !s->resident_ok)
     return set_error(AFL_ERR_INVALID_ARGUMENT,
                      "the %dx%dx%d grid does not fit the resident CG kernel", g.nx, g.ny, g.nz);
-  if (want_resident && s->brick_ok) {
+  if (want_resident && s->brick_ok && s->precision == AFL_PRECISION_FP64) {
     const afl::BrickSolve a{g, s->p, s->b, s->brick_scratch, iters, s->params.cg_rel_tol, rep,
                             s->ps.timeout_ns};
     blocks = afl::launch_cg_brick(a, s->brick, s->stream);
@@ -372,13 +372,20 @@ afl_status stage_solve(afl_solver *s, int kind, int iters, afl::SolveReport *rep
     a.rel_tol = s->params.cg_rel_tol;
     a.report = rep;
     blocks = afl::launch_cg_resident(a, s->resident, f64, s->ps, s->stream);
+  } else if (kind != AFL_POISSON_CG && s->brick_ok &&
+             s->params.poisson_kernel != AFL_POISSON_KERNEL_STREAMING) {
+    const afl::BrickSor a{g, s->p, s->b, s->brick_scratch, iters, s->params.sor_omega, rep,
+                          s->ps.timeout_ns};
+    blocks = afl::launch_sor_brick(a, s->brick, s->precision == AFL_PRECISION_FP64, s->stream);
+    abort_flag = static_cast<const int *>(s->brick_scratch);
   } else if (kind != AFL_POISSON_CG && s->resident_ok &&
              (s->params.poisson_kernel == AFL_POISSON_KERNEL_RESIDENT ||
               (s->params.poisson_kernel == AFL_POISSON_KERNEL_AUTO &&
                s->precision != AFL_PRECISION_FP64))) {
-    // RB-SOR on chip: the automatic choice for the mixed form only.  The FP64
-    // sweep re-reads its f64 right-hand side from L2 every half-sweep (no room
-    // on chip beside the f64 tile), and the streaming colour walk is faster.
+    // RB-SOR on column tiles, for grids that fit those but no bricks: the
+    // automatic choice for the mixed form only.  The FP64 sweep re-reads its f64
+    // right-hand side from L2 every half-sweep (no room on chip beside the f64
+    // tile), and the streaming colour walk is faster.
     const bool f64 = s->precision == AFL_PRECISION_FP64;
     afl::ResidentSorArgs a{};
     a.g = g;
@@ -680,8 +687,7 @@ afl_status afl_create(size_t nx, size_t ny, size_t nz, const afl_params *params,
   // one block: the resident FP64 CG reads cg[0..3] as four consecutive arrays,
   // the brick-resident one keeps its slots and inboxes there
   s->resident_ok = afl::plan_resident(s->g, s->precision == AFL_PRECISION_FP64, &s->resident);
-  s->brick_ok = s->resident_ok && s->precision == AFL_PRECISION_FP64 &&
-                afl::plan_brick(s->g, &s->brick);
+  s->brick_ok = s->resident_ok && afl::plan_brick(s->g, &s->brick);
   size_t cg_bytes = fb * static_cast<size_t>(ncg);
   if (s->brick_ok) cg_bytes = std::max(cg_bytes, afl::brick_scratch_bytes(s->brick));
   void *cg_block = nullptr;

@@ -1,8 +1,9 @@
-"""The brick-resident FP64 CG at the sizes where its bricks, faces and padding
-planes can go wrong, against the streaming kernel on the same system.  The two
-differ in the order of the sums and in the rounding of the fused updates, so 30
-iterations agree to 1e-10 of the pressure's norm (the bound the other resident
-kernels are held to)."""
+"""The brick-resident kernels at the sizes where their bricks, faces and padding
+planes can go wrong, against the streaming kernels on the same system.  The CG
+kernels differ in the order of the sums and in the rounding of the fused
+updates, so 30 iterations agree to 1e-10 of the pressure's norm (the bound the
+other resident kernels are held to).  An FP64 RB-SOR sweep reads only the other
+colour, so it is the same bits; the mixed sweep agrees to f32 rounding (1e-5)."""
 import numpy as np
 import pytest
 
@@ -79,3 +80,44 @@ def test_brick_stops_where_streaming_stops(af):
     z = np.zeros_like(b)
     got, gi = solve(af, shape, 0, z, z, 50)
     assert gi.converged and gi.iterations == 0 and not got.any()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", SHAPES, ids=["x".join(map(str, s)) for s in SHAPES])
+def test_brick_sor_matches_streaming(af, shape, precision):
+    b, p0 = system(shape, 9, True)
+    out = []
+    for kernel in (1, 0):
+        s = af.FluidSolver3D(*shape, precision=precision, poisson_kernel=kernel)
+        s.set_params(solver_kind=1, sor_omega=1.7)
+        s.set_field("divergence", b)
+        s.set_field("pressure", p0)
+        info = s.solve_poisson_gauss_seidel(9)
+        assert info.iterations == 9
+        out.append(s.get_field("pressure"))
+        s.close()
+    if precision == 0:
+        assert np.array_equal(out[0], out[1])
+    else:
+        assert rel_l2(out[1], out[0]) <= 1e-5
+
+
+def test_brick_sor_division_edges(af):
+    """Quotients whose numerators are zero, subnormal, huge, infinite or NaN are
+    the division's own."""
+    shape = (34, 20, 12)
+    nx, ny, nz = shape
+    rng = np.random.default_rng(3)
+    b = rng.standard_normal((nz, ny, nx))
+    scale = 10.0 ** rng.uniform(-320, 300, size=b.shape)
+    b = np.where(rng.random(b.shape) < 0.3, 0.0, b * scale)
+    b[5, 6, 7], b[8, 9, 30] = np.inf, np.nan
+    out = []
+    for kernel in (1, 0):
+        s = af.FluidSolver3D(*shape, poisson_kernel=kernel)
+        s.set_params(solver_kind=1, sor_omega=1.7)
+        s.set_field("divergence", b.ravel())
+        s.solve_poisson_gauss_seidel(1)
+        out.append(s.get_field("pressure"))
+        s.close()
+    assert np.array_equal(out[0], out[1], equal_nan=True)
