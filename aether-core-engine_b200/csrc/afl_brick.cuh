@@ -314,6 +314,9 @@ struct BrickFaces {
 };
 
 // ---- tensor memory as per-thread storage -------------------------------------------
+// Every load, store and wait below starts with __syncwarp(): the .sync.aligned
+// forms need the whole warp converged, and a branch that only some lanes took
+// just before does not promise that (an illegal instruction otherwise).
 // 128 lanes x 512 columns of 32 bits beside the register file and shared
 // memory.  Warp w reaches lanes 32*(w%4) .. +31 and owns a quarter of the
 // allocated columns; 32x32b loads and stores move a thread's own columns.
@@ -337,16 +340,19 @@ __device__ __forceinline__ void brick_tm_sync_threads() {
 }
 // 8 columns; asynchronous: brick_tm_wait_st before the next load of them.
 __device__ __forceinline__ void brick_tm_st8(unsigned taddr, const unsigned (&v)[8]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr),
       "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
       : "memory");
 }
 __device__ __forceinline__ void brick_tm_wait_st() {
+  __syncwarp();
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 // 16 columns; the registers are valid after brick_tm_wait_ld on them.
 __device__ __forceinline__ void brick_tm_ld16(unsigned taddr, unsigned (&v)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
@@ -358,6 +364,7 @@ __device__ __forceinline__ void brick_tm_ld16(unsigned taddr, unsigned (&v)[16])
 }
 // Names the registers, so that no use of them moves above the wait.
 __device__ __forceinline__ void brick_tm_wait_ld(unsigned (&v)[16]) {
+  __syncwarp();
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]),
                  "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]),
