@@ -237,6 +237,18 @@ struct BrickSor {
   unsigned long long timeout_ns;
 };
 int launch_sor_brick(const BrickSor &s, const BrickPlan &plan, bool f64, cudaStream_t st);
+// The mixed CG on the same bricks (afl_mixed_brick.cu); arguments as MixedCgArgs.
+struct BrickMixedSolve {
+  Dims g;
+  double *p;
+  const double *b;
+  void *scratch;
+  int max_total, max_inner, max_refine;
+  double inner_rel_tol, rel_tol;
+  SolveReport *report;
+  unsigned long long timeout_ns;
+};
+int launch_cg_brick_mixed(const BrickMixedSolve &s, const BrickPlan &plan, cudaStream_t st);
 // Returns the CTAs launched, or minus a cudaError_t.
 int launch_cg_brick(const BrickSolve &s, const BrickPlan &plan, cudaStream_t st);
 

@@ -351,7 +351,14 @@ afl_status stage_solve(afl_solver *s, int kind, int iters, afl::SolveReport *rep
       !s->resident_ok)
     return set_error(AFL_ERR_INVALID_ARGUMENT,
                      "the %dx%dx%d grid does not fit the resident CG kernel", g.nx, g.ny, g.nz);
-  if (want_resident && s->brick_ok && s->precision == AFL_PRECISION_FP64) {
+  if (want_resident && s->brick_ok && s->precision != AFL_PRECISION_FP64) {
+    const afl::BrickMixedSolve a{g, s->p, s->b, s->brick_scratch, std::max(1, iters),
+                                 std::max(1, s->params.mixed_inner_iters),
+                                 s->params.mixed_max_refinements, s->params.mixed_inner_rel_tol,
+                                 s->params.cg_rel_tol, rep, s->ps.timeout_ns};
+    blocks = afl::launch_cg_brick_mixed(a, s->brick, s->stream);
+    abort_flag = static_cast<const int *>(s->brick_scratch);
+  } else if (want_resident && s->brick_ok) {
     const afl::BrickSolve a{g, s->p, s->b, s->brick_scratch, iters, s->params.cg_rel_tol, rep,
                             s->ps.timeout_ns};
     blocks = afl::launch_cg_brick(a, s->brick, s->stream);

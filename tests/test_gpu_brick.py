@@ -2,7 +2,7 @@
 planes can go wrong, against the streaming kernels on the same system.  The CG
 kernels differ in the order of the sums and in the rounding of the fused
 updates, so 30 iterations agree to 1e-10 of the pressure's norm (the bound the
-other resident kernels are held to).  An FP64 RB-SOR sweep reads only the other
+other resident kernels are held to), of the mixed form's to 1e-4.  An FP64 RB-SOR sweep reads only the other
 colour, so it is the same bits; the mixed sweep agrees to f32 rounding (1e-5)."""
 import numpy as np
 import pytest
@@ -36,8 +36,9 @@ def system(shape, seed, walls):
     return b.ravel(), rng.standard_normal(nx * ny * nz) * 0.01
 
 
-def solve(af, shape, kernel, b, p0, iters, rel_tol=0.0):
-    s = af.FluidSolver3D(*shape, poisson_kernel=kernel, cg_rel_tol=rel_tol)
+def solve(af, shape, kernel, b, p0, iters, rel_tol=0.0, precision=0, **knobs):
+    s = af.FluidSolver3D(*shape, precision=precision, poisson_kernel=kernel, cg_rel_tol=rel_tol,
+                         **knobs)
     s.set_field("divergence", b)
     s.set_field("pressure", p0)
     info = s.solve_poisson_conjugate_gradient(iters)
@@ -66,6 +67,27 @@ def test_brick_wall_cells_of_the_right_hand_side(af, shape):
     got, gi = solve(af, shape, 0, b, p0, 3)
     assert gi.iterations == ri.iterations == 3
     assert rel_l2(got, ref) <= 1e-10
+
+
+@pytest.mark.parametrize("shape", SHAPES[1:], ids=["x".join(map(str, s)) for s in SHAPES[1:]])
+def test_brick_mixed_matches_streaming(af, shape):
+    b, p0 = system(shape, 7, False)
+    knobs = dict(precision=1, mixed_inner_iters=15, mixed_max_refinements=2)
+    ref, ri = solve(af, shape, 1, b, p0, 30, **knobs)
+    got, gi = solve(af, shape, 0, b, p0, 30, **knobs)
+    assert (gi.iterations, gi.refinements) == (ri.iterations, ri.refinements)
+    assert rel_l2(got, ref) <= 1e-4
+    assert abs(gi.final_residual - ri.final_residual) <= 1e-2 * ri.final_residual
+
+
+def test_brick_mixed_wall_cells_of_the_right_hand_side(af):
+    shape = (64, 64, 75)
+    b, p0 = system(shape, 5, True)
+    knobs = dict(precision=1, mixed_inner_iters=3, mixed_max_refinements=1)
+    ref, ri = solve(af, shape, 1, b, p0, 3, **knobs)
+    got, gi = solve(af, shape, 0, b, p0, 3, **knobs)
+    assert gi.iterations == ri.iterations == 3
+    assert rel_l2(got, ref) <= 1e-4
 
 
 def test_brick_stops_where_streaming_stops(af):
