@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/aether_fluid.h"
+#include "afl_host.h"
 #include "afl_launch.h"
 
 namespace afl {
@@ -378,6 +379,7 @@ afl_status upload(afl_adjoint *a, double *dst, const double *host) {
 }
 
 afl_status download(afl_adjoint *a, double *host, const double *src) {
+  afl::prefault(host, nbytes(a));
   ADJ_CUDA(cudaMemcpyAsync(host, src, nbytes(a), cudaMemcpyDeviceToHost, a->stream));
   ADJ_CUDA(cudaStreamSynchronize(a->stream));
   return AFL_OK;

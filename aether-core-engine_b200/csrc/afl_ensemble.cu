@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "../../include/aether_fluid.h"
+#include "afl_host.h"
 #include "afl_launch.h"
 
 namespace {
@@ -629,6 +630,7 @@ afl_status afl_ensemble_download_field(afl_ensemble *e, int instance, int field,
     return fail(AFL_ERR_INVALID_ARGUMENT, "bad field id");
   if (n != static_cast<size_t>(e->dims[instance].n))
     return fail(AFL_ERR_INVALID_ARGUMENT, "length does not match the instance grid");
+  afl::prefault(host, n * sizeof(double));
   ENS_CUDA(cudaStreamSynchronize(e->stream));
   void *src = nullptr;
   ENS_TRY(current_field(e, instance, field, &src));

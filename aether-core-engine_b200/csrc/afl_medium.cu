@@ -16,6 +16,7 @@
 #include <cstdio>
 
 #include "../../include/aether_fluid.h"
+#include "afl_host.h"
 #include "afl_launch.h"
 
 namespace afl {
@@ -382,6 +383,8 @@ afl_status afl_medium_sample_density_temp(afl_medium *m, const double *points, s
   const int ni = static_cast<int>(n);
   afl::k_medium_sample<<<(ni + afl::kMT - 1) / afl::kMT, afl::kMT, 0, m->stream>>>(m->dev, in, ni,
                                                                                   o, o + n);
+  afl::prefault(density, n * sizeof(double));
+  afl::prefault(temperature, n * sizeof(double));
   MED_CUDA(cudaMemcpyAsync(density, o, n * sizeof(double), cudaMemcpyDeviceToHost, m->stream));
   MED_CUDA(cudaMemcpyAsync(temperature, o + n, n * sizeof(double), cudaMemcpyDeviceToHost,
                            m->stream));
@@ -404,6 +407,7 @@ afl_status afl_medium_transmittance(afl_medium *m, const afl_ray *rays, size_t n
   const int ni = static_cast<int>(n);
   afl::k_medium_transmittance<<<(ni + afl::kMT - 1) / afl::kMT, afl::kMT, 0, m->stream>>>(
       m->dev, in, ni, static_cast<unsigned long long>(seed), o);
+  afl::prefault(transmittance, n * sizeof(double));
   MED_CUDA(cudaMemcpyAsync(transmittance, o, n * sizeof(double), cudaMemcpyDeviceToHost,
                            m->stream));
   return finish(m);
@@ -428,6 +432,8 @@ afl_status afl_medium_sample_interaction(afl_medium *m, const afl_ray *rays, siz
   const int ni = static_cast<int>(n);
   afl::k_medium_interaction<<<(ni + afl::kMT - 1) / afl::kMT, afl::kMT, 0, m->stream>>>(
       m->dev, in, ni, static_cast<unsigned long long>(seed), h, o, o + n, o + 2 * n);
+  afl::prefault(hit, n * sizeof(int32_t));
+  for (double *out : {t, density, temperature}) afl::prefault(out, n * sizeof(double));
   MED_CUDA(cudaMemcpyAsync(hit, h, n * sizeof(int32_t), cudaMemcpyDeviceToHost, m->stream));
   if (t) MED_CUDA(cudaMemcpyAsync(t, o, n * sizeof(double), cudaMemcpyDeviceToHost, m->stream));
   if (density)

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/aether_fluid.h"
+#include "afl_host.h"
 #include "afl_launch.h"
 
 using afl::Dims;
@@ -838,6 +839,7 @@ afl_status afl_download_field(afl_solver *s, int field, double *host, size_t n) 
   if (!host) return set_error(AFL_ERR_INVALID_ARGUMENT, "null host buffer");
   DeviceGuard guard(s->device);
   const size_t bytes = n * sizeof(double);
+  afl::prefault(host, bytes);
   const void *src = nullptr;
   if (field == AFL_FIELD_PRESSURE) {
     src = s->p;
@@ -1108,6 +1110,7 @@ afl_status afl_sample_trilinear(afl_solver *s, int field, const double *xyz, siz
   }
   s->launches += 1;
   AFL_TRY(launch_check());
+  afl::prefault(out, npts * sizeof(double));
   AFL_CUDA(cudaMemcpyAsync(out, d_out, npts * sizeof(double), cudaMemcpyDeviceToHost,
                            s->stream));
   return sync_and_check(s);
