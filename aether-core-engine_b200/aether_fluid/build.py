@@ -24,7 +24,7 @@ COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
           "--expt-relaxed-constexpr", "-extended-lambda"]
 # Units whose f64 arithmetic must not be contracted into FMAs.
 NO_FMA = {"afl_kernels_f64.cu", "afl_poisson_f64.cu", "afl_poisson_resident.cu",
-          "afl_poisson_brick.cu", "afl_sor_brick.cu", "afl_mixed_brick.cu",
+          "afl_poisson_brick.cu", "afl_sor_brick.cu", "afl_mixed_brick.cu", "afl_cg_sweep.cu",
           "afl_poisson_stream.cu", "afl_ensemble_f64.cu", "afl_ensemble_persist.cu",
           "afl_adjoint_kernels.cu", "afl_medium.cu"}
 SOURCES = [
@@ -36,6 +36,7 @@ SOURCES = [
     "afl_poisson_brick.cu",
     "afl_sor_brick.cu",
     "afl_mixed_brick.cu",
+    "afl_cg_sweep.cu",
     "afl_poisson_stream.cu",
     "afl_solver.cu",
     "afl_noalloc.cu",

@@ -271,6 +271,11 @@ int stream_vector_width(const Dims &g, bool f64);
 int launch_cg_stream_f64(const CgArgs &a, const PersistentState &ps, cudaStream_t st);
 int launch_cg_stream_mixed(const MixedCgArgs &a, const PersistentState &ps, cudaStream_t st);
 int persistent_blocks_stream();
+// The streaming CG at one sweep per iteration (afl_cg_sweep.cu), for grids whose
+// vectors leave L2 and whose rows are 16-byte aligned.  ps.partials holds the sums' slots.
+bool sweep_fits(const Dims &g, bool f64);
+int launch_cg_sweep_f64(const CgArgs &a, const PersistentState &ps, cudaStream_t st);
+int launch_cg_sweep_mixed(const MixedCgArgs &a, const PersistentState &ps, cudaStream_t st);
 
 // One system of the batched (multi-grid) streaming CG: its arguments, its own
 // barrier and partials (2 buffers x 3 values x ctas), and its CTA range.

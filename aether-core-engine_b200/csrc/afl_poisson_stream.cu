@@ -1,5 +1,7 @@
 // afl_poisson_stream.cu -- streaming persistent CG for grids that do not fit
-// on chip (256^3 and up), vectorised along x.
+// on chip, vectorised along x, in two passes per iteration.  Grids whose vectors
+// leave L2 and whose rows are aligned take one sweep per iteration instead
+// (afl_cg_sweep.cu).
 //
 // Each thread handles runs of V consecutive x cells (the widest of 4 / 2 / 1
 // doubles or 8 / 4 / 1 floats that divides nx) and walks the runs of the
@@ -140,6 +142,8 @@ int stream_vector_width(const Dims &g, bool f64) {
 }
 
 int launch_cg_stream_f64(const CgArgs &a, const PersistentState &ps, cudaStream_t st) {
+  if (sweep_fits(a.g, true))
+    if (const int blocks = launch_cg_sweep_f64(a, ps, st)) return blocks;
   switch (stream_vector_width(a.g, true)) {
     case 4: return launch_persistent(&k_cg_stream_f64<4>, a, ps, 2, st);
     case 2: return launch_persistent(&k_cg_stream_f64<2>, a, ps, 2, st);
@@ -148,6 +152,8 @@ int launch_cg_stream_f64(const CgArgs &a, const PersistentState &ps, cudaStream_
 }
 
 int launch_cg_stream_mixed(const MixedCgArgs &a, const PersistentState &ps, cudaStream_t st) {
+  if (sweep_fits(a.g, false))
+    if (const int blocks = launch_cg_sweep_mixed(a, ps, st)) return blocks;
   switch (stream_vector_width(a.g, false)) {
     case 8: return launch_persistent(&k_cg_stream_mixed<8>, a, ps, 3, st);
     case 4: return launch_persistent(&k_cg_stream_mixed<4>, a, ps, 3, st);

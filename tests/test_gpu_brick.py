@@ -143,3 +143,53 @@ def test_brick_sor_division_edges(af):
         out.append(s.get_field("pressure"))
         s.close()
     assert np.array_equal(out[0], out[1], equal_nan=True)
+
+
+# Beyond the chip and L2 CG makes one sweep per iteration (aligned rows): tiles of 128
+# and of 32, one and several chunks, ragged edges, odd and even sweep counts, against
+# numpy's f64 CG.  Five steps on a random right-hand side: f64 rounds at 1e-15 a step,
+# f32 at 1e-6.
+SWEEP_SHAPES = [(160, 160, 161), (130, 250, 126), (256, 140, 118), (194, 66, 322), (250, 300, 44)]
+
+
+def numpy_cg(shape, b, p, iters):
+    nx, ny, nz = shape
+    sl = (slice(1, -1),) * 3
+    b, p = b.reshape(nz, ny, nx)[sl], p.reshape(nz, ny, nx)[sl].copy()
+
+    def nb(x):
+        s = np.zeros_like(x)
+        for a in range(3):
+            lo = tuple(slice(None, -1) if q == a else slice(None) for q in range(3))
+            hi = tuple(slice(1, None) if q == a else slice(None) for q in range(3))
+            s[hi] += x[lo]
+            s[lo] += x[hi]
+        return s
+
+    diag = nb(np.ones_like(p))
+    r = b - (diag * p - nb(p))
+    d, delta = r.copy(), float(np.vdot(r, r))
+    for _ in range(iters):
+        q = diag * d - nb(d)
+        alpha = delta / float(np.vdot(d, q))
+        p += alpha * d
+        r -= alpha * q
+        new = float(np.vdot(r, r))
+        d = r + new / delta * d
+        delta = new
+    return p, np.sqrt(delta)
+
+
+@pytest.mark.parametrize("precision,tol", [(0, 1e-10), (1, 1e-4)])
+@pytest.mark.parametrize("shape", SWEEP_SHAPES, ids=["x".join(map(str, s)) for s in SWEEP_SHAPES])
+@pytest.mark.parametrize("iters", [4, 5])
+def test_sweep_matches_numpy(af, shape, precision, tol, iters):
+    if precision:  # twice the cells before f32 vectors leave L2
+        shape = (256, 192, 2 * shape[2])
+    b, p0 = system(shape, 11, False)
+    got, info = solve(af, shape, 1, b, p0, iters, precision=precision, mixed_max_refinements=1)
+    want, res = numpy_cg(shape, b, p0, iters)
+    assert info.iterations == iters
+    inner = got.reshape(shape[::-1])[1:-1, 1:-1, 1:-1]
+    assert rel_l2(inner.ravel(), want.ravel()) <= tol
+    assert abs(info.final_residual - res) <= (1e-9 if precision == 0 else 1e-3) * res
