@@ -632,7 +632,10 @@ constexpr int kRingScalar = 6, kRingForces = 6;
 
 // z planes per CTA: about four waves of two resident CTAs per SM over the
 // grid, and at least 8 planes per CTA (the ring is primed with two planes
-// below the chunk).
+// below the chunk).  A grid that does not fill one wave that way takes as few as 2
+// planes per CTA to fill it: its time is one CTA's march, and the planes staged twice
+// come from L2 (us, scalars / forces: 36 x 52 x 36 with jets, 9 -> 2 planes, 65 -> 27 /
+// 16.5 -> 9.3).
 inline int fused_kz(const Dims &g) {
   const int ctas_per_sm = 2;
   const int tiles = ((g.nx + kFx - 1) / kFx) * ((g.ny + kFy - 1) / kFy);
@@ -647,6 +650,11 @@ inline int fused_kz(const Dims &g) {
   long chunks = (want + tiles - 1) / tiles;
   const long max_chunks = g.nz / 8 > 0 ? g.nz / 8 : 1;
   if (chunks > max_chunks) chunks = max_chunks;
+  const long wave = static_cast<long>(sms) * ctas_per_sm;
+  if (tiles * chunks < wave) {
+    const long thin = g.nz / 2 > 0 ? g.nz / 2 : 1;
+    chunks = wave / tiles < thin ? wave / tiles : thin;
+  }
   if (chunks < 1) chunks = 1;
   return static_cast<int>((g.nz + chunks - 1) / chunks);
 }

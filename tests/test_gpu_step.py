@@ -245,3 +245,19 @@ def test_odd_grid_plume_matches_oracle(af, oracle, solver, precision, tol):
     for f in ("u", "v", "w", "density", "temperature"):
         err = rel_l2(s.get_field(f), o.field(f))
         assert err <= tol, (f, err)
+
+
+@pytest.mark.parametrize("shape", [(8, 9, 7), (33, 17, 7), (36, 52, 36), (64, 24, 61)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_thin_plane_chunks_bit_exact(af, oracle, shape):
+    """Grids whose fused stages march 2 to 7 planes per CTA, some with a ragged last
+    chunk: 3 steps of an RB-SOR plume, fixed-order arithmetic except telemetry, bit for
+    bit."""
+    from aether_fluid.plume import Plume
+    p = Plume(*shape, 3, seed=5, solver="sor", iters=20)
+    o = oracle_for(p, oracle)
+    o.run(p.steps, p.dt, 0.0, p.dt)
+    s = p.build()
+    s.run(p.steps, p.dt, 0.0, p.dt)
+    for f in FIELDS:
+        assert np.array_equal(s.get_field(f), o.field(f)), f
