@@ -129,6 +129,13 @@ struct BrickSums {
   __device__ __forceinline__ Packet *of(unsigned tag) const {
     return slots + static_cast<size_t>(tag & 1u) * 4 * nblocks;
   }
+  __device__ __forceinline__ int block() const { return static_cast<int>(blockIdx.x); }
+};
+// ... of one system of several in a launch (afl_launch.h, BrickQueue): this CTA is
+// block vblock of it.
+struct QueuedSums : BrickSums {
+  int vblock;
+  __device__ __forceinline__ int block() const { return vblock; }
 };
 
 // First half of publishing a sum: warp sums of v (a butterfly that halves the
@@ -162,14 +169,13 @@ __device__ __forceinline__ double brick_cta_sum(const double *red) {
 
 // Second half: warp 0 publishes the CTA's partials as sum number `tag`.
 // RELEASE: also releases the CTA's writes before the barrier.
-template <bool RELEASE>
-__device__ __forceinline__ void brick_publish(const BrickSums &bs, unsigned tag,
-                                              const double *red) {
+template <bool RELEASE, typename Sums>
+__device__ __forceinline__ void brick_publish(const Sums &bs, unsigned tag, const double *red) {
   if (threadIdx.x >= 32) return;
   const double y = brick_cta_sum(red);
   if (threadIdx.x < 4) {
     if (RELEASE) __threadfence();
-    st_packet(bs.of(tag) + blockIdx.x * 4 + threadIdx.x, y, tag);
+    st_packet(bs.of(tag) + bs.block() * 4 + threadIdx.x, y, tag);
   }
 }
 
@@ -228,9 +234,9 @@ struct BrickCells {
   int i, j, z0, nzb;     // column; first plane; planes of the brick inside the grid
   bool in_ij;
   int c0;                // global index of the column's cell in plane 0
-  __device__ __forceinline__ BrickCells(const Dims &g, int nbx, int nby, int cz, int t) {
-    bx = blockIdx.x % nbx;
-    const int q = blockIdx.x / nbx;
+  __device__ __forceinline__ BrickCells(const Dims &g, int nbx, int nby, int cz, int t, int block) {
+    bx = block % nbx;
+    const int q = block / nbx;
     by = q % nby;
     bz = q / nby;
     i = bx * S::BX + t % S::BX;
@@ -312,6 +318,112 @@ struct BrickFaces {
     side_d = m0 * S::SXY + (rj + 1) * S::SX + ri + 1;
   }
 };
+
+// ---- several systems in one launch ---------------------------------------------------
+// Bricks are kQueueBX wide for every system, and an inbox belongs to a CTA, not to a
+// system: a CTA leaves a system only after it has read every packet sent to it, and
+// clears its inbox before the next one's first sum.
+constexpr int kQueueBX = 16;
+
+template <typename Args>
+struct BrickJob {
+  Args a;
+  BrickSums bs;
+  int begin;  // the system's first CTA
+};
+
+template <typename Args>
+struct BrickQueue {
+  const BrickJob<Args> *jobs;
+  const int *first, *list;
+};
+
+// Where the parts of the queue's scratch start.
+struct QueueLayout {
+  size_t first, list, slots, inbox, bytes;
+  QueueLayout(const BrickQueuePlan &q, size_t job_bytes, size_t packet_bytes) {
+    auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+    first = up(job_bytes * q.plan.size());
+    list = first + sizeof(int) * q.first.size();
+    slots = up(list + sizeof(int) * q.list.size());
+    inbox = up(slots + sizeof(Packet) * 8 * static_cast<size_t>(q.total));
+    czp = q.cz_class;
+    bytes = inbox + 2 * packet_bytes * per() * static_cast<size_t>(q.ctas);
+  }
+  int czp = 0;
+  size_t per() const {
+    return static_cast<size_t>(brick_inbox_packets(BrickShape<kQueueBX>::kSide, czp));
+  }
+};
+
+// The jobs and lists on the device; fill(m, args) sets system m's own arguments.
+template <typename Args, typename Mem, typename Fill>
+cudaError_t write_queue(const BrickQueuePlan &q, void *scratch, int *abort_flag,
+                        unsigned long long timeout_ns, Fill fill) {
+  using Job = BrickJob<Args>;
+  const QueueLayout at(q, sizeof(Job), sizeof(Mem));
+  auto *const base = static_cast<unsigned char *>(scratch);
+  std::vector<Job> jobs(q.plan.size());
+  size_t slot = 0;
+  for (size_t m = 0; m < jobs.size(); ++m) {
+    const BrickPlan &p = q.plan[m];
+    Args &a = jobs[m].a;
+    fill(m, a);
+    a.nbx = p.nbx;
+    a.nby = p.nby;
+    a.nbz = p.nbz;
+    a.cz = p.cz;
+    a.czp = q.cz_class;
+    a.inbox = reinterpret_cast<Mem *>(base + at.inbox) + at.per() * static_cast<size_t>(q.begin[m]);
+    a.parity = static_cast<int>(at.per() * static_cast<size_t>(q.ctas));
+    jobs[m].bs = BrickSums{reinterpret_cast<Packet *>(base + at.slots) + 8 * slot, p.ctas(),
+                           abort_flag, timeout_ns};
+    jobs[m].begin = q.begin[m];
+    slot += static_cast<size_t>(p.ctas());
+  }
+  auto put = [&](size_t off, const void *src, size_t bytes) {
+    return cudaMemcpy(base + off, src, bytes, cudaMemcpyHostToDevice);
+  };
+  cudaError_t err = put(0, jobs.data(), sizeof(Job) * jobs.size());
+  if (err == cudaSuccess) err = put(at.first, q.first.data(), sizeof(int) * q.first.size());
+  if (err == cudaSuccess) err = put(at.list, q.list.data(), sizeof(int) * q.list.size());
+  return err;
+}
+
+template <typename Args, typename Mem, typename Fn>
+int launch_queue(Fn fn, size_t smem, const BrickQueuePlan &q, void *scratch, cudaStream_t st) {
+  const QueueLayout at(q, sizeof(BrickJob<Args>), sizeof(Mem));
+  auto *const base = static_cast<unsigned char *>(scratch);
+  const void *const f = reinterpret_cast<const void *>(fn);
+  cudaError_t err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+  if (err != cudaSuccess) return -static_cast<int>(err);
+  cudaMemsetAsync(base + at.slots, 0, sizeof(Packet) * 8 * static_cast<size_t>(q.total), st);
+  BrickQueue<Args> a{reinterpret_cast<const BrickJob<Args> *>(base),
+                     reinterpret_cast<const int *>(base + at.first),
+                     reinterpret_cast<const int *>(base + at.list)};
+  void *params[] = {&a};
+  err = cudaLaunchCooperativeKernel(f, dim3(q.ctas), dim3(kBT), params, smem, st);
+  return err == cudaSuccess ? q.ctas : -static_cast<int>(err);
+}
+
+// This CTA's systems in order: solve(args, sums) of each, from shared memory.
+template <typename Args, typename Solve>
+__device__ __forceinline__ void run_queue(const BrickQueue<Args> &q, Args &a, QueuedSums &bs,
+                                          Solve solve) {
+  const int end = q.first[blockIdx.x + 1];
+  for (int n = q.first[blockIdx.x]; n < end; ++n) {
+    __syncthreads();  // the previous system's shared memory is free
+    if (threadIdx.x == 0) {
+      const BrickJob<Args> &job = q.jobs[q.list[n]];
+      a = job.a;
+      static_cast<BrickSums &>(bs) = job.bs;
+      bs.vblock = static_cast<int>(blockIdx.x) - job.begin;
+    }
+    __syncthreads();
+    solve();
+  }
+}
 
 // ---- tensor memory as per-thread storage -------------------------------------------
 // Every load, store and wait below starts with __syncwarp(): the .sync.aligned

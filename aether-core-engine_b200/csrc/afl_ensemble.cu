@@ -3,13 +3,15 @@
 //
 // Every stage of a step is one batched launch over all instances (block table
 // -> instance descriptor -> the single-grid per-cell code), and the pressure
-// solves of all instances run in one cooperative launch whose CTAs are split
-// between the instances (afl_poisson_stream.cu, k_cg_stream_multi).  One step
-// is captured once into a CUDA graph and replayed.  By default the whole step
-// instead runs as one persistent cooperative launch (afl_ensemble_persist.cu),
-// itself captured in the graph; it measured 0-5 % faster on the 48-plume
-// ensemble.  The autotuner chooses the CTA split of the
-// solve by timing candidate splits on a snapshot of the state, which it then
+// solves of all instances run in one cooperative launch: on chip, each CTA
+// working through a list of bricks (afl_brick.cuh, plan_brick_queue), or, where
+// that is not faster, streaming with the CTAs split between the instances
+// (afl_poisson_stream.cu, k_cg_stream_multi).  One step is captured once into a
+// CUDA graph and replayed.  By default the stages instead run as one persistent
+// cooperative launch before and one after the solve, or one around a streaming
+// solve (afl_ensemble_persist.cu), captured in the graph too.  The autotuner
+// chooses the stages' CTA split (with a streaming solve, the solve's too) and
+// tile depth by timing candidates on a snapshot of the state, which it then
 // restores.
 #include <cuda_runtime.h>
 
@@ -129,6 +131,8 @@ struct afl_ensemble {
   afl::MultiCgSystem *d_sys = nullptr;
   int *d_cta_inst = nullptr;
   int total_ctas = 0;
+  afl::BrickQueuePlan brick;      // the solves on chip
+  void *brick_scratch = nullptr;  // null: the streaming solve above
   unsigned int *d_bar = nullptr;  // count/gen per instance + shared abort flag
   double *d_cg_partials = nullptr;
   // graph
@@ -322,6 +326,36 @@ afl_status build_systems(afl_ensemble *e, const std::vector<int> &ctas) {
   return AFL_OK;
 }
 
+// The solves on chip, where that is faster; without the memory for it they stream.
+afl_status build_bricks(afl_ensemble *e) {
+  if (!afl::plan_brick_queue(e->dims, std::max(1, e->common.solver_iters), e->f64, &e->brick)) return AFL_OK;
+  void *scratch = nullptr;
+  if (cudaMalloc(&scratch, afl::brick_queue_scratch_bytes(e->brick, e->f64)) != cudaSuccess) {
+    cudaGetLastError();
+    return AFL_OK;
+  }
+  e->allocs.push_back(scratch);
+  int *const abort_flag = reinterpret_cast<int *>(e->d_bar + 2 * e->count);
+  const unsigned long long timeout_ns = 5000000000ull;
+  std::vector<afl::BrickSolve> f64;
+  std::vector<afl::BrickMixedSolve> mixed;
+  const afl_params &c = e->common;
+  for (int m = 0; m < e->count; ++m) {
+    const Bufs &B = e->bufs[m];
+    if (e->f64)
+      f64.push_back({e->dims[m], B.p, B.b, nullptr, c.solver_iters, c.cg_rel_tol,
+                     e->d_rep_cur + m, 0});
+    else
+      mixed.push_back({e->dims[m], B.p, B.b, nullptr, std::max(1, c.solver_iters),
+                       std::max(1, c.mixed_inner_iters), c.mixed_max_refinements,
+                       c.mixed_inner_rel_tol, c.cg_rel_tol, e->d_rep_cur + m, 0});
+  }
+  ENS_CUDA(e->f64 ? afl::setup_brick_queue(f64, e->brick, scratch, abort_flag, timeout_ns)
+                  : afl::setup_brick_queue(mixed, e->brick, scratch, abort_flag, timeout_ns));
+  e->brick_scratch = scratch;
+  return AFL_OK;
+}
+
 template <typename T>
 afl_status enqueue_step(afl_ensemble *e) {
   afl::EnsLaunch<T> L{static_cast<afl::EnsInstance<T> *>(e->d_inst), e->d_blk_inst, e->blocks,
@@ -330,8 +364,15 @@ afl_status enqueue_step(afl_ensemble *e) {
   if (e->persistent) {
     ENS_CUDA(cudaMemsetAsync(e->d_bar, 0, sizeof(unsigned int) * (2 * e->count + 1), st));
     afl::EnsStepArgs a{e->d_inst, e->d_sys,       e->d_cta_inst, e->d_tel_partials, e->d_step,
-                       e->d_tel_out, e->d_rep_cur, e->d_reports,  e->count,          e->capacity};
-    const int used = afl::launch_ens_step(a, e->f64, e->vec, e->total_ctas, st);
+                       e->d_tel_out, e->d_rep_cur, e->d_reports,  e->count,          e->capacity, 0};
+    int used = 1;
+    if (e->brick_scratch) {
+      a.phase = 1;
+      used = afl::launch_ens_step(a, e->f64, e->vec, e->total_ctas, st);
+      if (used > 0) used = afl::launch_cg_brick_queue(e->brick, e->f64, e->brick_scratch, st);
+      a.phase = 2;
+    }
+    if (used > 0) used = afl::launch_ens_step(a, e->f64, e->vec, e->total_ctas, st);
     if (used <= 0) return cuda_fail(static_cast<cudaError_t>(-used), "persistent step launch");
     afl::ens_step_advance(e->d_step, st);
     ENS_CUDA(cudaGetLastError());
@@ -344,7 +385,10 @@ afl_status enqueue_step(afl_ensemble *e) {
   afl::ens_forces<T>(L, st);  // sphere source + curl + confinement/buoyancy/wall BC
   afl::ens_divergence<T>(L, st);
   ENS_CUDA(cudaMemsetAsync(e->d_bar, 0, sizeof(unsigned int) * (2 * e->count + 1), st));
-  const int used = afl::launch_cg_multi(e->d_sys, e->d_cta_inst, e->total_ctas, e->f64, e->vec, st);
+  const int used =
+      e->brick_scratch
+          ? afl::launch_cg_brick_queue(e->brick, e->f64, e->brick_scratch, st)
+          : afl::launch_cg_multi(e->d_sys, e->d_cta_inst, e->total_ctas, e->f64, e->vec, st);
   if (used <= 0)
     return cuda_fail(static_cast<cudaError_t>(-used), "batched pressure solve launch");
   afl::ens_project<T>(L, st);
@@ -558,6 +602,7 @@ afl_status afl_ensemble_create(const afl_instance *inst, int count, const afl_pa
   // the persistent step is the default form when every instance gets a CTA
   e->persistent = e->budget_step >= count;
   st = build_systems(e, split_ctas(w, active_budget(e)));
+  if (st == AFL_OK) st = build_bricks(e);
   if (st == AFL_OK) st = ensure_capacity(e, 1);
   if (st != AFL_OK) return bail(st);
   if (!e->graph_ok) build_graph(e);

@@ -18,11 +18,14 @@
 // therefore round each product and sum separately here, where the batched
 // f32 kernels may contract them.
 //
+// A solve that runs on chip has its own launch; the step is then one launch of this
+// kernel before it and one after it (phase).
+//
 // Every stage runs at the solve's occupancy (4 CTAs per SM at 64 registers;
 // 5 per SM spills 300-480 bytes), and the solve gets 592 CTAs instead of the
 // graph form's 740.  Its CG body therefore prefetches the runs two steps ahead
-// into L2.  Measured on the 48-plume ensemble (mixed, 100 steps, autotuned):
-// 645-650 Mcell-steps/s against 632-633 for the graph of stage launches (593
+// into L2.  Measured with streaming solves on the 48-plume ensemble (mixed, 100 steps,
+// autotuned): 645-650 Mcell-steps/s against 632-633 for the graph of stage launches (593
 // without the prefetch), so this is the default form.
 #define AFL_RESTRICT
 #include <type_traits>
@@ -61,6 +64,11 @@ __global__ void __launch_bounds__(kST, kStepCtasPerSm) kp_ens_step(EnsStepArgs a
     }
     __syncthreads();
   };
+  auto keep_fields = [&] {
+    EnsInstance<T> &out = static_cast<EnsInstance<T> *>(a.inst)[m];
+    for (int f = 0; f < 5; ++f) out.fld[f] = d.fld[f];
+    out.tmp_out = d.tmp_out;
+  };
   auto advect = [&](int f, double diss) {
     each([&](int lb) { blk_advect_fwd(d, lb, f); });
     if (!grid_sync(gs)) return false;
@@ -69,25 +77,33 @@ __global__ void __launch_bounds__(kST, kStepCtasPerSm) kp_ens_step(EnsStepArgs a
     swap_out(f);
     return true;
   };
-  for (int f = 0; f < 3; ++f)
-    if (!advect(f, 0.996)) return;
-  each([&](int lb) { blk_curl(d, lb); });
-  if (!grid_sync(gs)) return;
-  each([&](int lb) { blk_source_confine_buoy(d, lb); });
-  if (!grid_sync(gs)) return;
-  each([&](int lb) { blk_divergence(d, lb); });
-  if (!grid_sync(gs)) return;
-  bool ok;
-  if constexpr (std::is_same<T, double>::value) {
-    const Ring3 pr{s.partials, 2 * nv};
-    ok = cg_stream_f64_body<V, false, true>(s.f64, gs, pr, vb, nv, scratch);
-  } else {
-    const Ring3 pr{s.partials, 3 * nv};
-    ok = cg_stream_mixed_body<V, false, true>(s.mixed, gs, pr, vb, nv, scratch);
+  if (a.phase != 2) {
+    for (int f = 0; f < 3; ++f)
+      if (!advect(f, 0.996)) return;
+    each([&](int lb) { blk_curl(d, lb); });
+    if (!grid_sync(gs)) return;
+    each([&](int lb) { blk_source_confine_buoy(d, lb); });
+    if (!grid_sync(gs)) return;
+    each([&](int lb) { blk_divergence(d, lb); });
+    if (!grid_sync(gs)) return;
   }
-  // The solve ends at a barrier after its last pressure write; this one also
-  // separates its last read of the partials from the stages' writes.
-  if (!ok || !grid_sync(gs)) return;
+  if (a.phase == 0) {
+    bool ok;
+    if constexpr (std::is_same<T, double>::value) {
+      const Ring3 pr{s.partials, 2 * nv};
+      ok = cg_stream_f64_body<V, false, true>(s.f64, gs, pr, vb, nv, scratch);
+    } else {
+      const Ring3 pr{s.partials, 3 * nv};
+      ok = cg_stream_mixed_body<V, false, true>(s.mixed, gs, pr, vb, nv, scratch);
+    }
+    // The solve ends at a barrier after its last pressure write; this one also
+    // separates its last read of the partials from the stages' writes.
+    if (!ok || !grid_sync(gs)) return;
+  }
+  if (a.phase == 1) {
+    if (vb == 0 && threadIdx.x == 0) keep_fields();
+    return;
+  }
   each([&](int lb) { blk_project(d, lb); });
   if (!grid_sync(gs)) return;
   if (!advect(3, 0.996)) return;
@@ -99,11 +115,7 @@ __global__ void __launch_bounds__(kST, kStepCtasPerSm) kp_ens_step(EnsStepArgs a
   if (vb == 0) {
     ens_finalize(d, m, a.tel_partials, step, a.tel_out, a.rep_cur, a.reports, a.count,
                  a.capacity, scratch);
-    if (threadIdx.x == 0) {
-      EnsInstance<T> &out = static_cast<EnsInstance<T> *>(a.inst)[m];
-      for (int f = 0; f < 5; ++f) out.fld[f] = d.fld[f];
-      out.tmp_out = d.tmp_out;
-    }
+    if (threadIdx.x == 0) keep_fields();
   }
 }
 

@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "afl_device.cuh"
 
 struct afl_solver;  // include/aether_fluid.h
@@ -249,6 +251,28 @@ struct BrickMixedSolve {
   unsigned long long timeout_ns;
 };
 int launch_cg_brick_mixed(const BrickMixedSolve &s, const BrickPlan &plan, cudaStream_t st);
+// Several systems in one launch (the ensembles), each on its own run of CTAs; a CTA
+// takes the systems of its list in order.  Lists that follow one order of all
+// systems cannot deadlock: the first unfinished system has all its CTAs.
+struct BrickQueuePlan {
+  int cz_class = 0;              // planes a CTA holds at most: 4, 8, 16 or 32
+  int ctas = 0;                  // of the launch
+  int total = 0;                 // over all systems (slots are 8 packets each)
+  std::vector<BrickPlan> plan;   // per system; only the shape
+  std::vector<int> begin;        // its first CTA
+  std::vector<int> first, list;  // CTA c takes systems list[first[c] .. first[c + 1])
+};
+// False when some system needs more bricks than SMs, or streaming is the faster.
+bool plan_brick_queue(const std::vector<Dims> &g, int max_iters, bool f64, BrickQueuePlan *plan);
+size_t brick_queue_scratch_bytes(const BrickQueuePlan &plan, bool f64);
+// Writes the jobs of the solves s (their scratch and timeouts unset) into scratch.
+cudaError_t setup_brick_queue(const std::vector<BrickSolve> &s, const BrickQueuePlan &plan,
+                              void *scratch, int *abort_flag, unsigned long long timeout_ns);
+cudaError_t setup_brick_queue(const std::vector<BrickMixedSolve> &s, const BrickQueuePlan &plan,
+                              void *scratch, int *abort_flag, unsigned long long timeout_ns);
+int launch_cg_brick_queue(const BrickQueuePlan &plan, bool f64, void *scratch, cudaStream_t st);
+size_t mixed_queue_scratch_bytes(const BrickQueuePlan &plan);  // the f32 halves of these two
+int launch_cg_brick_queue_mixed(const BrickQueuePlan &plan, void *scratch, cudaStream_t st);
 // Returns the CTAs launched, or minus a cudaError_t.
 int launch_cg_brick(const BrickSolve &s, const BrickPlan &plan, cudaStream_t st);
 
@@ -345,6 +369,8 @@ struct EnsStepArgs {
   const SolveReport *rep_cur;
   SolveReport *reports;
   int count, capacity;
+  int phase;                  // 0: the whole step; 1, 2: the stages before and after a
+                              // solve of its own launch
 };
 // Co-resident CTAs of the step kernel for the precision and run width v.
 int persistent_blocks_ens_step(bool f64, int v);

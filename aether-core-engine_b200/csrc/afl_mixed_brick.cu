@@ -49,8 +49,8 @@ __device__ __forceinline__ double mixed_residual(const Dims &g, const double *p,
   return b[c] - (diag * __ldcg(p + c) - nb);
 }
 
-template <int BX, int CZ>
-__device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, const BrickSums &bs,
+template <int BX, int CZ, typename Sums>
+__device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, const Sums &bs,
                                                     float *D, double *red, double *keep) {
   using S = BrickShape<BX>;
   constexpr bool SM = CZ > 8;             // e in shared memory, else in registers
@@ -61,7 +61,7 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
   const Dims &g = a.g;
   const int t = threadIdx.x;
   const int cz = a.cz;
-  const BrickCells<S> cl(g, a.nbx, a.nby, cz, t);
+  const BrickCells<S> cl(g, a.nbx, a.nby, cz, t, bs.block());
   const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp);
   const int k0 = cl.z0, k_lo = 2 - k0, k_hi = min(g.nz - 3 - k0, cl.nzb - 1);
   const bool col_in = cl.column_interior(g);
@@ -242,7 +242,7 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
           }
         }
         if (!col_in) acc[0] = acc[1] = acc[2] = 0.0;
-        if (blockIdx.x == 0 && t == 0) acc[3] += keep[3];
+        if (bs.block() == 0 && t == 0) acc[3] += keep[3];
       }
       brick_partials(acc, red);
       if (fc.xdst >= 0) {
@@ -367,7 +367,7 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
     ++passes;
     if (rr < 1e-20 || (keep[2] >= 0.0 && rr <= keep[2])) converged = 1;
   }
-  if (blockIdx.x == 0 && t == 0 && a.report) {
+  if (bs.block() == 0 && t == 0 && a.report) {
     SolveReport rep;
     rep.iterations = total;
     rep.refinements = passes;
@@ -387,6 +387,16 @@ __global__ void __launch_bounds__(kBT, 1)
   extern __shared__ float Fsm[];
   __shared__ double red[2 * 4 * kBW], keep[6];
   cg_brick_mixed_body<BX, CZ>(a, bs, Fsm, red, keep);
+}
+
+template <int CZ>
+__global__ void __launch_bounds__(kBT, 1)
+    k_cg_brick_queue_mixed(const __grid_constant__ BrickQueue<BrickMixedArgs> q) {
+  extern __shared__ float Fsm[];
+  __shared__ double red[2 * 4 * kBW], keep[6];
+  __shared__ BrickMixedArgs a;
+  __shared__ QueuedSums bs;
+  run_queue(q, a, bs, [&] { cg_brick_mixed_body<kQueueBX, CZ>(a, bs, Fsm, red, keep); });
 }
 
 using BrickMixedFn = void (*)(BrickMixedArgs, BrickSums);
@@ -438,6 +448,35 @@ int launch_cg_brick_mixed(const BrickMixedSolve &s, const BrickPlan &plan, cudaS
   err = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fn), dim3(blocks), dim3(kBT),
                                     params, smem, st);
   return err == cudaSuccess ? blocks : -static_cast<int>(err);
+}
+
+cudaError_t setup_brick_queue(const std::vector<BrickMixedSolve> &s, const BrickQueuePlan &plan,
+                              void *scratch, int *abort_flag, unsigned long long timeout_ns) {
+  return write_queue<BrickMixedArgs, unsigned long long>(
+      plan, scratch, abort_flag, timeout_ns, [&](size_t m, BrickMixedArgs &a) {
+        a.g = s[m].g;
+        a.p = s[m].p;
+        a.b = s[m].b;
+        a.max_total = s[m].max_total;
+        a.max_inner = s[m].max_inner;
+        a.max_refine = s[m].max_refine;
+        a.inner_rel_tol = s[m].inner_rel_tol;
+        a.rel_tol = s[m].rel_tol;
+        a.report = s[m].report;
+      });
+}
+
+size_t mixed_queue_scratch_bytes(const BrickQueuePlan &plan) {
+  return QueueLayout(plan, sizeof(BrickJob<BrickMixedArgs>), sizeof(unsigned long long)).bytes;
+}
+
+int launch_cg_brick_queue_mixed(const BrickQueuePlan &q, void *scratch, cudaStream_t st) {
+  const auto fn = q.cz_class == 4    ? &k_cg_brick_queue_mixed<4>
+                  : q.cz_class == 8  ? &k_cg_brick_queue_mixed<8>
+                  : q.cz_class == 16 ? &k_cg_brick_queue_mixed<16>
+                                     : &k_cg_brick_queue_mixed<32>;
+  return launch_queue<BrickMixedArgs, unsigned long long>(fn, mixed_smem<kQueueBX>(q.cz_class), q,
+                                                          scratch, st);
 }
 
 }  // namespace afl

@@ -31,6 +31,8 @@
 // extra words crowd the lines being waited for).
 //
 // Built with -fmad=false; the FMAs of the solve are written out (__fma_rn).
+#include <algorithm>
+#include <numeric>
 #include <type_traits>
 
 #include "afl_brick.cuh"
@@ -79,8 +81,8 @@ __device__ __forceinline__ double brick_residual(const Dims &g, const double *p,
 // p gains b times the sum of alpha_k s_k.  Their r.r joins the sums as one
 // number, and p gets its gain at the end (b is 0 there after a divergence; a
 // caller's own right-hand side may not be).
-template <int BX, int CZ>
-__device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const BrickSums &bs,
+template <int BX, int CZ, typename Sums>
+__device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Sums &bs,
                                                   double *D, double *red, double *keep, unsigned tm) {
   using S = BrickShape<BX>;
   constexpr bool TM = CZ > 8;             // q and p in tensor memory, else in registers
@@ -91,7 +93,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Br
   const Dims &g = a.g;
   const int t = threadIdx.x;
   const int cz = a.cz;
-  const BrickCells<S> cl(g, a.nbx, a.nby, cz, t);
+  const BrickCells<S> cl(g, a.nbx, a.nby, cz, t, bs.block());
   const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp);
   // z of the brick's plane m is k0 + m; chunks whose four planes all have both
   // z neighbours take the plain path of the operator
@@ -297,7 +299,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Br
       double q_lo, q_hi, q_side[NI], sum[4];
       bool ok = true;
       {
-        const Packet *const own = box + blockIdx.x * brick_inbox_packets(S::kSide, a.czp) + t;
+        const Packet *const own = box + bs.block() * brick_inbox_packets(S::kSide, a.czp) + t;
         RawPacket lo, hi, side[NI];
         const int side_lim = I[kSide] & 255;
         const bool zlo = I[kZlo] >= 0, zhi = I[kZhi] >= 0;
@@ -365,7 +367,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Br
       if (t == 0) {
         keep[5] += alpha * keep[4];
         keep[4] = 1.0 + beta * keep[4];
-        if (blockIdx.x == 0) rr = keep[3];
+        if (bs.block() == 0) rr = keep[3];
       }
       auto update = [&](int m, double q, double &p) {
         const double dv = Dc[m * SXY];
@@ -409,7 +411,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Br
   // ---- the pressure back to global memory ----------------------------------------
   int t2;
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t2));  // kept apart: no register across the loop
-  const BrickCells<S> cw(g, a.nbx, a.nby, cz, t2);
+  const BrickCells<S> cw(g, a.nbx, a.nby, cz, t2, bs.block());
   __syncthreads();
   const bool wall = keep[3] != 0.0;
   const double gain = keep[5];
@@ -434,7 +436,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Br
       }
     }
   }
-  if (blockIdx.x == 0 && t2 == 0 && a.report) {
+  if (bs.block() == 0 && t2 == 0 && a.report) {
     SolveReport rep;
     rep.iterations = it;
     rep.refinements = 0;
@@ -466,6 +468,31 @@ __global__ void __launch_bounds__(kBT, 1)
     if (warp == 0) brick_tm_dealloc<COLS>(tm_base);
   } else {
     cg_brick_f64_body<BX, CZ>(a, bs, Dsm, red, keep, 0u);
+  }
+}
+
+// Several systems, each CTA its list of them.
+template <int CZ>
+__global__ void __launch_bounds__(kBT, 1)
+    k_cg_brick_queue_f64(const __grid_constant__ BrickQueue<BrickCgArgs> q) {
+  extern __shared__ double Dsm[];
+  __shared__ double red[2 * 4 * kBW], keep[6];
+  __shared__ unsigned tm_base;
+  __shared__ BrickCgArgs a;
+  __shared__ QueuedSums bs;
+  constexpr bool TM = CZ > 8;
+  constexpr int COLS = 16 * CZ;
+  const int warp = threadIdx.x >> 5;
+  unsigned tm = 0;
+  if constexpr (TM) {
+    if (warp == 0) brick_tm_alloc<COLS>(&tm_base);
+    brick_tm_sync_threads();
+    tm = tm_base + ((32u * unsigned(warp & 3)) << 16) + unsigned(4 * CZ) * unsigned(warp >> 2);
+  }
+  run_queue(q, a, bs, [&] { cg_brick_f64_body<kQueueBX, CZ>(a, bs, Dsm, red, keep, tm); });
+  if constexpr (TM) {
+    brick_tm_sync_threads();
+    if (warp == 0) brick_tm_dealloc<COLS>(tm_base);
   }
 }
 
@@ -562,6 +589,119 @@ int launch_cg_brick(const BrickSolve &s, const BrickPlan &plan, cudaStream_t st)
   err = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fn), dim3(blocks), dim3(kBT),
                                     params, plan.smem_bytes, st);
   return err == cudaSuccess ? blocks : -static_cast<int>(err);
+}
+
+// Planes per CTA: the fewest of 4, 8, 16, 32 at which all systems run side by side, else up
+// to 32 and several systems per CTA.  Largest first, each where it can start earliest.
+// A solve is taken to need 3.5 iterations per cell of its longest side (32^3 115, 48^3 165).
+//
+// Against the streaming solve, which takes every system at once at 6.6 ps a cell and
+// iteration (FP64 13) and not less than 4 us an iteration.  ms per step, streaming -> this:
+// the 48 plumes 16.2 -> 11.3 (FP64 31.4 -> 11.9), one 32^3 1.6 -> 0.44, one 128^3 5.2 -> 2.4,
+// 140 of 16^3 1.6 -> 0.9, 9 of 96^3 13.2 -> 11.0; several per CTA on bricks that the grids
+// leave half empty lose in f32: 40 of 40^3 3.8 -> 4.5 (FP64 5.2 -> 4.5), 300 of 16^3
+// 2.0 -> 2.2 (2.5 -> 2.2).
+bool plan_brick_queue(const std::vector<Dims> &g, int max_iters, bool f64, BrickQueuePlan *q) {
+  using S = BrickShape<kQueueBX>;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  sms = std::min(sms, 160);
+  const int count = static_cast<int>(g.size());
+  for (q->cz_class = 4;; q->cz_class *= 2) {
+    q->plan.clear();
+    q->total = 0;
+    int most = 0;
+    for (const Dims &d : g) {
+      BrickPlan p{};
+      p.bx = S::BX;
+      p.nbx = (d.nx + S::BX - 1) / S::BX;
+      p.nby = (d.ny + S::BY - 1) / S::BY;
+      const int layers = (d.nz + q->cz_class - 1) / q->cz_class;
+      p.cz = (d.nz + layers - 1) / layers;
+      p.nbz = (d.nz + p.cz - 1) / p.cz;
+      if (static_cast<long long>(p.nbx) * p.nby * p.nbz > sms) most = sms + 1;
+      else q->total += p.ctas(), most = std::max(most, p.ctas());
+      q->plan.push_back(p);
+    }
+    if (most <= sms && q->total <= sms) break;
+    if (q->cz_class == kBrickMaxPlanes) {
+      if (most > sms) return false;
+      break;
+    }
+  }
+  std::vector<int> order(count);
+  std::iota(order.begin(), order.end(), 0);
+  int most_planes = 0;
+  for (const BrickPlan &p : q->plan) most_planes = std::max(most_planes, p.cz);
+  q->cz_class = brick_cz_class(most_planes);
+  auto iterations = [&](int m) {
+    return std::min(double(max_iters), 3.5 * std::max(g[m].nx, std::max(g[m].ny, g[m].nz)));
+  };
+  auto cost = [&](int m) { return iterations(m) * 0.2 * (12 + q->plan[m].cz); };  // us
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return cost(a) * q->plan[a].ctas() > cost(b) * q->plan[b].ctas();
+  });
+  std::vector<double> free(sms, 0.0);
+  std::vector<std::vector<int>> lists(sms);
+  q->begin.assign(count, 0);
+  q->ctas = 0;
+  for (int m : order) {
+    const int n = q->plan[m].ctas();
+    double best = 0.0;
+    for (int b = 0; b + n <= sms; ++b) {
+      const double at = *std::max_element(free.begin() + b, free.begin() + b + n);
+      if (b > 0 && at >= best) continue;
+      best = at;
+      q->begin[m] = b;
+    }
+    for (int c = q->begin[m]; c < q->begin[m] + n; ++c) {
+      free[c] = best + cost(m);
+      lists[c].push_back(m);
+    }
+    q->ctas = std::max(q->ctas, q->begin[m] + n);
+  }
+  double cells = 0.0, longest = 0.0;
+  for (int m = 0; m < count; ++m) {
+    cells += iterations(m) * g[m].n;
+    longest = std::max(longest, iterations(m));
+  }
+  const double streaming = cells * (f64 ? 13e-6 : 6.6e-6) + longest * 4.0;
+  if (*std::max_element(free.begin(), free.end()) > streaming) return false;
+  q->first.assign(1, 0);
+  q->list.clear();
+  for (int c = 0; c < q->ctas; ++c) {
+    q->list.insert(q->list.end(), lists[c].begin(), lists[c].end());
+    q->first.push_back(static_cast<int>(q->list.size()));
+  }
+  return true;
+}
+
+cudaError_t setup_brick_queue(const std::vector<BrickSolve> &s, const BrickQueuePlan &plan,
+                              void *scratch, int *abort_flag, unsigned long long timeout_ns) {
+  return write_queue<BrickCgArgs, Packet>(plan, scratch, abort_flag, timeout_ns,
+                                          [&](size_t m, BrickCgArgs &a) {
+                                            a.g = s[m].g;
+                                            a.p = s[m].p;
+                                            a.b = s[m].b;
+                                            a.max_iters = s[m].max_iters;
+                                            a.rel_tol = s[m].rel_tol;
+                                            a.report = s[m].report;
+                                          });
+}
+
+size_t brick_queue_scratch_bytes(const BrickQueuePlan &plan, bool f64) {
+  return f64 ? QueueLayout(plan, sizeof(BrickJob<BrickCgArgs>), sizeof(Packet)).bytes
+             : mixed_queue_scratch_bytes(plan);
+}
+
+int launch_cg_brick_queue(const BrickQueuePlan &q, bool f64, void *scratch, cudaStream_t st) {
+  if (!f64) return launch_cg_brick_queue_mixed(q, scratch, st);
+  const auto fn = q.cz_class == 4    ? &k_cg_brick_queue_f64<4>
+                  : q.cz_class == 8  ? &k_cg_brick_queue_f64<8>
+                  : q.cz_class == 16 ? &k_cg_brick_queue_f64<16>
+                                     : &k_cg_brick_queue_f64<32>;
+  return launch_queue<BrickCgArgs, Packet>(fn, brick_smem<kQueueBX>(q.cz_class), q, scratch, st);
 }
 
 }  // namespace afl
