@@ -336,7 +336,13 @@ afl_status build_bricks(afl_ensemble *e) {
   }
   e->allocs.push_back(scratch);
   int *const abort_flag = reinterpret_cast<int *>(e->d_bar + 2 * e->count);
-  const unsigned long long timeout_ns = 5000000000ull;
+  // a system's first sum also waits for CTAs that are still at the systems before it
+  // (an iteration takes 3 to 10 us)
+  unsigned long long turns = 0;
+  for (int c = 0; c < e->brick.ctas; ++c)
+    turns = std::max<unsigned long long>(turns, e->brick.first[c + 1] - e->brick.first[c]);
+  const unsigned long long timeout_ns =
+      5000000000ull + (turns - 1) * 50000ull * std::max(1, e->common.solver_iters);
   std::vector<afl::BrickSolve> f64;
   std::vector<afl::BrickMixedSolve> mixed;
   const afl_params &c = e->common;
