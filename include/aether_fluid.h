@@ -74,13 +74,16 @@ typedef enum afl_precision {
 } afl_precision;
 
 /* Poisson kernel choice.  CG, AUTO: an on-chip resident kernel when the grid
- * fits (tiles <= SMs, tile + halo in shared memory; FP64 runs in bricks where
+ * fits (tiles <= SMs, tile + halo in shared memory; it runs in bricks where
  * the grid also splits into no more 512-column bricks than SMs, else in column
- * tiles), else the streaming kernel; they differ only in the summation order of
- * the inner products and in the rounding of fused updates.
- * RB-SOR, AUTO: the resident kernel for the mixed form when the grid fits,
- * else the streaming sweep; RESIDENT selects the resident sweep for FP64 too
- * (same result bit for bit, since a colour reads only the other colour). */
+ * tiles), else a streaming kernel (one sweep over memory per iteration where the
+ * vectors leave L2 and the rows are 16-byte aligned, else two passes); they
+ * differ only in the summation order of the inner products and in the rounding
+ * of fused updates.
+ * RB-SOR, AUTO: bricks where the grid fits those, else the column-tile kernel
+ * for the mixed form when the grid fits it, else the streaming sweep; RESIDENT
+ * selects the column tiles for FP64 too (same result bit for bit, since a
+ * colour reads only the other colour). */
 typedef enum afl_poisson_kernel {
   AFL_POISSON_KERNEL_AUTO = 0,
   AFL_POISSON_KERNEL_STREAMING = 1,
@@ -287,7 +290,8 @@ afl_status afl_ensemble_run(afl_ensemble *e, int steps, afl_telemetry *telemetry
                             afl_solve_info *infos);
 afl_status afl_ensemble_download_field(afl_ensemble *e, int instance, int field, double *host,
                                        size_t n);
-/* Picks the CTA split of the batched solve by timing candidates on a snapshot
+/* Picks the CTA split of the persistent stages and of a streaming batched solve
+ * (a solve on chip has its own) and the tile depth by timing candidates on a snapshot
  * of the state (restored afterwards); *choice gets the candidate index. */
 afl_status afl_ensemble_autotune(afl_ensemble *e, int32_t *choice);
 /* out = {instances, step graph captured (1/0), solver CTAs, co-resident CTA
@@ -299,8 +303,9 @@ afl_status afl_ensemble_instance_ctas(const afl_ensemble *e, int32_t *out, int c
  * the solver's CTA split; these set and read it directly. */
 afl_status afl_ensemble_set_tile_depth(afl_ensemble *e, int32_t kz);
 afl_status afl_ensemble_tile_depth(const afl_ensemble *e, int32_t *kz);
-/* Step form: 1 = one persistent cooperative launch per step, the CTAs of
- * each instance meeting at the instance's own bounded barrier between stages
+/* Step form: 1 = the stages as one persistent cooperative launch before and one
+ * after the on-chip solve (one around a streaming solve), the CTAs of each
+ * instance meeting at the instance's own bounded barrier between stages
  * (the default when the step kernel's co-resident CTAs outnumber the
  * instances); 0 = the captured graph of per-stage batched launches plus the
  * cooperative solve.  Setting it re-splits the CTAs for the form's
