@@ -39,6 +39,7 @@ namespace {
 
 constexpr int kSY = 16;     // tile rows, a warp each
 constexpr int kAhead = 2;   // planes staged ahead of the one being computed
+static_assert(kAhead == 2, "a unit starts with groups -1 and 0; a barrier takes one at a time");
 constexpr int kDSlots = 3 + kAhead, kRSlots = 1 + kAhead, kNSlots = 3;
 
 // NC cells per thread, 32 apart in x: tiles of 32 * NC x 16 cells.
