@@ -122,6 +122,7 @@ struct BoundedWait {
 // read all of sum k, and k+2 only after every CTA published k+1, so the two
 // halves never mix.  Slots start at 0, tags at 1.
 struct BrickSums {
+  static constexpr bool kQueued = false;
   Packet *slots;
   int nblocks;
   int *abort_flag;
@@ -134,6 +135,7 @@ struct BrickSums {
 // ... of one system of several in a launch (afl_launch.h, BrickQueue): this CTA is
 // block vblock of it.
 struct QueuedSums : BrickSums {
+  static constexpr bool kQueued = true;
   int vblock;
   __device__ __forceinline__ int block() const { return vblock; }
 };
@@ -219,6 +221,25 @@ struct BrickShape {
   static constexpr int kSide = 2 * (BX + BY);             // side ring cells per plane
   static constexpr int kLanes = kBT / kSide;              // planes the ring threads cover at once
   static constexpr int kXLanes = kBT / (2 * BY);          // planes the x-face senders cover at once
+  // Offsets at which the CG kernels send face values (-1: not sent), from those of
+  // BrickFaces: a y face's plane m, the n-th staged x value of thread t; and whether a
+  // thread's n-th side ring cell is waited for.  In a queue a CTA sends exactly what is
+  // waited for: a packet that nobody reads could land after its receiver has gone on to
+  // another system and cleared its inbox for that one.  A launch with one system has no
+  // such next one, and sends the planes between nzb and the chunk's end as well: the
+  // test costs it 3 % of an iteration of 128^3 (mixed 9 %).
+  template <bool QUEUED>
+  static __host__ __device__ __forceinline__ int y_at(int ydst, int m, int nzb) {
+    return ydst >= 0 && (!QUEUED || m < nzb) ? ydst + m * kSide : -1;
+  }
+  template <bool QUEUED>
+  static __host__ __device__ __forceinline__ int x_at(int xdst, int t, int n, int cz, int nzb) {
+    return xdst >= 0 && t / (2 * BY) + n * kXLanes < (QUEUED ? nzb : cz)
+               ? xdst + n * kXLanes * kSide : -1;
+  }
+  static __host__ __device__ __forceinline__ bool side_on(int n, int side_lim) {
+    return n * kLanes < side_lim;
+  }
 };
 
 // Packets of one CTA's inbox for one parity: kSide per plane (x-, x+, y-, y+
@@ -234,7 +255,8 @@ struct BrickCells {
   int i, j, z0, nzb;     // column; first plane; planes of the brick inside the grid
   bool in_ij;
   int c0;                // global index of the column's cell in plane 0
-  __device__ __forceinline__ BrickCells(const Dims &g, int nbx, int nby, int cz, int t, int block) {
+  __host__ __device__ __forceinline__ BrickCells(const Dims &g, int nbx, int nby, int cz, int t,
+                                                 int block) {
     bx = block % nbx;
     const int q = block / nbx;
     by = q % nby;
@@ -242,7 +264,7 @@ struct BrickCells {
     i = bx * S::BX + t % S::BX;
     j = by * S::BY + t / S::BX;
     z0 = bz * cz;
-    nzb = min(cz, g.nz - z0);
+    nzb = cz < g.nz - z0 ? cz : g.nz - z0;
     in_ij = i < g.nx && j < g.ny;
     c0 = (z0 * g.ny + j) * g.nx + i;
   }
@@ -274,9 +296,8 @@ struct BrickFaces {
   int side_lim;       // the thread's n-th side ring cell exists when n * kLanes < side_lim
   int side_d;         // its shared index in D for n = 0
   int si, sj;         // column of the side ring position
-  __device__ __forceinline__ BrickFaces(const Dims &g, const BrickCells<S> &cl, int nbx, int nby,
-                                        int nbz, int czp) {
-    const int t = threadIdx.x;
+  __host__ __device__ __forceinline__ BrickFaces(const Dims &g, const BrickCells<S> &cl, int nbx,
+                                                 int nby, int nbz, int czp, int t) {
     const int ii = t % S::BX, jj = t / S::BX;
     const int per = brick_inbox_packets(S::kSide, czp);
     auto box = [&](int dx, int dy, int dz) {
@@ -290,6 +311,7 @@ struct BrickFaces {
       const int xs = t % (2 * S::BY), m0 = t / (2 * S::BY) * S::kSide;
       xdst = xs < S::BY ? (cl.bx > 0 ? box(-1, 0, 0) + S::BY + xs + m0 : -1)
                         : (cl.bx + 1 < nbx ? box(1, 0, 0) + xs - S::BY + m0 : -1);
+      if (cl.by * S::BY + xs % S::BY >= g.ny) xdst = -1;  // a row past the grid
     }
     xcol = -1;
     if (cl.in_ij) {
@@ -321,8 +343,9 @@ struct BrickFaces {
 
 // ---- several systems in one launch ---------------------------------------------------
 // Bricks are kQueueBX wide for every system, and an inbox belongs to a CTA, not to a
-// system: a CTA leaves a system only after it has read every packet sent to it, and
-// clears its inbox before the next one's first sum.
+// system: a CTA leaves a system only after it has read every packet sent to it (none is
+// sent that is not waited for: BrickShape::y_at, x_at), and clears its inbox before the
+// next one's first sum.
 constexpr int kQueueBX = 16;
 
 template <typename Args>

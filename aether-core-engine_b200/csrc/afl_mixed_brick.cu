@@ -62,7 +62,7 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
   const int t = threadIdx.x;
   const int cz = a.cz;
   const BrickCells<S> cl(g, a.nbx, a.nby, cz, t, bs.block());
-  const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp);
+  const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp, t);
   const int k0 = cl.z0, k_lo = 2 - k0, k_hi = min(g.nz - 3 - k0, cl.nzb - 1);
   const bool col_in = cl.column_interior(g);
   const bool side_in = fc.si >= 1 && fc.si <= g.nx - 2 && fc.sj >= 1 && fc.sj <= g.ny - 2;
@@ -229,7 +229,9 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
           if (fc.ydst >= 0) {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              st_packet(box + fc.ydst + (4 * ch + e) * S::kSide, q[4 * ch + e], tag);
+              if (const int at = S::template y_at<Sums::kQueued>(fc.ydst, 4 * ch + e, cl.nzb);
+                  at >= 0)
+                st_packet(box + at, q[4 * ch + e], tag);
           }
           if (ch == 0 && fc.zlo_dst >= 0) st_packet(box + fc.zlo_dst, q[0], tag);
           if (4 * ch + 4 >= cz && fc.zhi_dst >= 0) {
@@ -248,8 +250,8 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
       if (fc.xdst >= 0) {
 #pragma unroll
         for (int n = 0; n < CZ / S::kXLanes || n == 0; ++n)
-          if (t / XSTEP + n * S::kXLanes < cz)
-            st_packet(box + fc.xdst + n * S::kXLanes * S::kSide, X[t + n * kBT], tag);
+          if (const int at = S::template x_at<Sums::kQueued>(fc.xdst, t, n, cz, cl.nzb); at >= 0)
+            st_packet(box + at, X[t + n * kBT], tag);
       }
       brick_publish<false>(bs, tag, red);
       // ---- the ring's q, then the grid-wide sum ----------------------------------------
@@ -263,7 +265,7 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
           hi.ld(fc.zhi_dst >= 0, own + S::kSide * a.czp + kBT, tag);
 #pragma unroll
           for (int n = 0; n < NI; ++n)
-            side[n].ld(n * S::kLanes < fc.side_lim, own + n * RSTEP, tag);
+            side[n].ld(S::side_on(n, fc.side_lim), own + n * RSTEP, tag);
           bool got = lo.has(tag) & hi.has(tag);
 #pragma unroll
           for (int n = 0; n < NI; ++n) got &= side[n].has(tag);

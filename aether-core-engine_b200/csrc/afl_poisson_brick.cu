@@ -94,7 +94,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Su
   const int t = threadIdx.x;
   const int cz = a.cz;
   const BrickCells<S> cl(g, a.nbx, a.nby, cz, t, bs.block());
-  const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp);
+  const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp, t);
   // z of the brick's plane m is k0 + m; chunks whose four planes all have both
   // z neighbours take the plain path of the operator
   const int k0 = cl.z0, k_lo = 2 - k0, k_hi = min(g.nz - 3 - k0, cl.nzb - 1);
@@ -265,7 +265,8 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Su
           if (ydst >= 0) {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              st_packet(box + ydst + (4 * ch + e) * S::kSide, qv[e], tag);
+              if (const int at = S::template y_at<Sums::kQueued>(ydst, 4 * ch + e, cl.nzb); at >= 0)
+                st_packet(box + at, qv[e], tag);
           }
           if (ch == 0) {
             const int zlo = I[kZlo];
@@ -291,8 +292,8 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Su
       if (const int xdst = I[kXdst]; xdst >= 0) {
 #pragma unroll
         for (int n = 0; n < CZ / S::kXLanes || n == 0; ++n)
-          if (t / XSTEP + n * S::kXLanes < cz)
-            st_packet(box + xdst + n * S::kXLanes * S::kSide, X[t + n * kBT], tag);
+          if (const int at = S::template x_at<Sums::kQueued>(xdst, t, n, cz, cl.nzb); at >= 0)
+            st_packet(box + at, X[t + n * kBT], tag);
       }
       brick_publish<false>(bs, tag, red);
       // ---- the ring's q, the neighbours' packets, then the grid-wide sum --------
@@ -308,7 +309,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Su
           lo.ld(zlo, own + S::kSide * a.czp, tag);
           hi.ld(zhi, own + S::kSide * a.czp + kBT, tag);
 #pragma unroll
-          for (int n = 0; n < NI; ++n) side[n].ld(n * S::kLanes < side_lim, own + n * RSTEP, tag);
+          for (int n = 0; n < NI; ++n) side[n].ld(S::side_on(n, side_lim), own + n * RSTEP, tag);
           bool got = lo.has(tag) & hi.has(tag);
 #pragma unroll
           for (int n = 0; n < NI; ++n) got &= side[n].has(tag);

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kBT, 1) k_sor_brick(const __grid_constant__ Br
   const int t = threadIdx.x;
   const int cz = a.cz;
   const BrickCells<S> cl(g, a.nbx, a.nby, cz, t, static_cast<int>(blockIdx.x));
-  const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp);
+  const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp, t);
   T *const Pc = P + (t / S::BX + 1) * S::SX + t % S::BX + 1;
   T *const Z = P + (CZ + 1) * SXY + t;  // the cell below the column
   const int k0 = cl.z0, k_lo = 2 - k0, k_hi = min(g.nz - 3 - k0, cl.nzb - 1);
