@@ -33,11 +33,12 @@
 
 #include "afl_brick.cuh"
 #include "afl_cg_stream_body.cuh"
+#include "afl_sweep_plan.h"
 
 namespace afl {
 namespace {
 
-constexpr int kSY = 16;     // tile rows, a warp each
+constexpr int kSY = kSweepRows;
 constexpr int kAhead = 2;   // planes staged ahead of the one being computed
 static_assert(kAhead == 2, "a unit starts with groups -1 and 0; a barrier takes one at a time");
 constexpr int kDSlots = 3 + kAhead, kRSlots = 1 + kAhead, kNSlots = 3;
@@ -103,11 +104,6 @@ template <typename T>
 struct SweepVecs {
   T *r[2], *d[2];  // by sweep parity
   T *x;            // the solution
-};
-
-struct SweepPlan {
-  int tiles_x, tiles_y, chunks, depth;  // z chunks of `depth` planes
-  __host__ __device__ int units() const { return tiles_x * tiles_y * chunks; }
 };
 
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -620,27 +616,6 @@ int sweep_ctas(const void *fn) {
   return std::min(sms * per_sm, kBT);
 }
 
-// z chunks: the fewest that make the longest CTA's march shortest, counted in plane
-// steps of its units, each with its fill (320 x 256 x 200 in tiles of 32: 160 tiles on
-// 296 CTAs leave half the chip idle in one chunk).
-SweepPlan sweep_plan(const Dims &g, int nc, int ctas) {
-  constexpr long long kFill = 6;
-  SweepPlan pl;
-  pl.tiles_x = (g.nx + 32 * nc - 1) / (32 * nc);
-  pl.tiles_y = (g.ny + kSY - 1) / kSY;
-  const long long tiles = static_cast<long long>(pl.tiles_x) * pl.tiles_y;
-  long long best = 0;
-  for (int chunks = 1; chunks <= (g.nz + 15) / 16; ++chunks) {
-    const int depth = (g.nz + chunks - 1) / chunks;
-    const long long steps = (tiles * ((g.nz + depth - 1) / depth) + ctas - 1) / ctas * (depth + kFill);
-    if (best != 0 && steps >= best) continue;
-    best = steps;
-    pl.depth = depth;
-  }
-  pl.chunks = (g.nz + pl.depth - 1) / pl.depth;
-  return pl;
-}
-
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -668,15 +643,19 @@ bool encode(EncodeTiled fn, CUtensorMap *map, const Dims &g, T *base, int rows) 
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// 0 when there are no tensor maps for it (the caller keeps the two-pass kernel).
+// 0 when the sweep does not pay, or there are no tensor maps for it (the caller keeps the
+// two-pass kernel).
 template <typename T, int NC, typename Args>
 int launch_sweep(const void *fn, Args a, const PersistentState &ps, cudaStream_t st) {
   int ctas = sweep_ctas<T, NC>(fn);
   // the sums' slots take the place of the streaming kernels' partials
   ctas = std::min(ctas, static_cast<int>(12 * sizeof(double) * size_t(ps.max_blocks) /
                                          (8 * sizeof(Packet))));
+  if (ctas < 1) return 0;
+  a.plan = sweep_plan(a.g, NC, ctas);
+  if (!sweep_pays(a.g, a.plan, NC, ctas, sizeof(T) == 8)) return 0;
   const EncodeTiled enc = encode_tiled();
-  bool ok = ctas >= 1 && enc;
+  bool ok = enc != nullptr;
   for (int q = 0; q < 2 && ok; ++q)
     ok = encode<T, NC>(enc, &a.maps.r[q], a.g, a.v.r[q], kSY + 2) &&
          encode<T, NC>(enc, &a.maps.d[q], a.g, a.v.d[q], kSY + 4);
@@ -685,7 +664,6 @@ int launch_sweep(const void *fn, Args a, const PersistentState &ps, cudaStream_t
     cudaGetLastError();
     return 0;
   }
-  a.plan = sweep_plan(a.g, NC, ctas);
   const int blocks = std::min(ctas, a.plan.units());
   cudaMemsetAsync(ps.abort_flag, 0, sizeof(int), st);
   cudaMemsetAsync(ps.partials, 0, sizeof(Packet) * 8 * static_cast<size_t>(blocks), st);
@@ -696,34 +674,19 @@ int launch_sweep(const void *fn, Args a, const PersistentState &ps, cudaStream_t
   return err == cudaSuccess ? blocks : -static_cast<int>(err);
 }
 
-// Tiles 128 cells wide (4 per thread) unless the last one would be mostly empty (us per
-// iteration, tiles of 32 -> of 128: FP64 256 x 256 x 256 177 -> 153, 320 x 256 x 200
-// 173 -> 161, 220^3 110 -> 112; 200 x 300 x 300 207 -> 216, 192 x 300 x 300 173 -> 207).
-bool wide(const Dims &g) { return (g.nx + 127) / 128 * 128 <= 1.27 * g.nx; }
-
 }  // namespace
 
-// Rows and planes of the TMA boxes must be 16-byte aligned, and the sweep pays once
-// the vectors leave L2 (us per iteration, two passes -> sweep): FP64 160^3 57 -> 51,
-// 192 x 160 x 176 73 -> 66, 150 x 300 x 300 193 -> 146, 220^3 136 -> 112, 256^3 208 -> 153;
-// mixed 220^3 79 -> 70, 256 x 200 x 256 86 -> 73, 256^3 108 -> 87.  Below that the two
-// passes run from L2 and the sweep's chain per plane shows: FP64 64^3 15 -> 28,
-// 136 x 140 x 144 41 -> 40; mixed 192^3 50 -> 52, 160^3 33 -> 45.  f32 rows are half as
-// long in bytes: only full tiles pay (192 x 300 x 300 112 -> 120).
 bool sweep_fits(const Dims &g, bool f64) {
   int dev = 0, l2 = 0;
-  if (g.n > (1 << 30)) return false;  // cell indices stay clear of 2^31
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
   cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
-  // r, q, d twice and the solution; f32 once four of them do
-  const size_t bytes = (f64 ? 5 * sizeof(double) : 4 * sizeof(float)) * static_cast<size_t>(g.n);
-  return g.nx % (f64 ? 2 : 4) == 0 && bytes > static_cast<size_t>(l2) && (f64 || wide(g));
+  return sweep_fits(g, f64, static_cast<size_t>(l2));
 }
 
 int launch_cg_sweep_f64(const CgArgs &a, const PersistentState &ps, cudaStream_t st) {
   SweepCgArgs s{{}, a.g, {}, {{a.r, a.q}, {a.d0, a.d1}, a.p}, a.b, a.max_iters, a.rel_tol,
                 a.report};
-  if (wide(a.g))
+  if (sweep_wide(a.g))
     return launch_sweep<double, 4>(reinterpret_cast<const void *>(&k_cg_sweep_f64<4>), s, ps, st);
   return launch_sweep<double, 1>(reinterpret_cast<const void *>(&k_cg_sweep_f64<1>), s, ps, st);
 }

@@ -296,7 +296,8 @@ int launch_cg_stream_f64(const CgArgs &a, const PersistentState &ps, cudaStream_
 int launch_cg_stream_mixed(const MixedCgArgs &a, const PersistentState &ps, cudaStream_t st);
 int persistent_blocks_stream();
 // The streaming CG at one sweep per iteration (afl_cg_sweep.cu), for grids whose
-// vectors leave L2 and whose rows are 16-byte aligned.  ps.partials holds the sums' slots.
+// vectors leave L2 and whose rows are 16-byte aligned; the launches return 0 where its
+// tiles would be too empty to pay (afl_sweep_plan.h).  ps.partials holds the sums' slots.
 bool sweep_fits(const Dims &g, bool f64);
 int launch_cg_sweep_f64(const CgArgs &a, const PersistentState &ps, cudaStream_t st);
 int launch_cg_sweep_mixed(const MixedCgArgs &a, const PersistentState &ps, cudaStream_t st);
