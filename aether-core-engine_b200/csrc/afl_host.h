@@ -5,7 +5,7 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <system_error>
+#include <exception>
 #include <thread>
 
 #include <sys/mman.h>
@@ -52,7 +52,7 @@ inline void prefault(void *buf, size_t bytes) {
   int started = 1;
   try {
     for (; started < parts; ++started) others[started - 1] = std::thread(part, started);
-  } catch (const std::system_error &) {  // no thread to be had: the copy faults the rest
+  } catch (const std::exception &) {  // no thread or no memory for one: the copy faults the rest
   }
   part(0);
   for (int n = 1; n < started; ++n) others[n - 1].join();

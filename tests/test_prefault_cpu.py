@@ -45,3 +45,44 @@ def test_prefault_keeps_contents(tmp_path):
                            str(exe), "-lpthread"])
     out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
+
+
+NO_MEMORY = r"""
+#include "afl_host.h"
+#include <cstdio>
+#include <cstdlib>
+#include <new>
+// The allocation number `fail_at` from here on throws.
+static int fail_at = -1;
+void *operator new(size_t n) {
+  if (fail_at >= 0 && fail_at-- == 0) throw std::bad_alloc();
+  if (void *p = std::malloc(n)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
+int main() {
+  for (int at = 0; at < 4; ++at) {
+    const size_t n = size_t(70) << 20;
+    char *p = static_cast<char *>(mmap(nullptr, n, PROT_READ | PROT_WRITE,
+                                       MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
+    fail_at = at;
+    afl::prefault(p, n);
+    fail_at = -1;
+    munmap(p, n);
+  }
+  puts("ok");
+}
+"""
+
+
+def test_prefault_without_host_memory_for_its_threads(tmp_path):
+    """No exception leaves it and no thread is left unjoined, whichever thread's state cannot
+    be allocated: it is called from the C entries."""
+    src, exe = tmp_path / "n.cpp", tmp_path / "n"
+    src.write_text(NO_MEMORY)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-I",
+                           os.path.join(ROOT, "aether-core-engine_b200", "csrc"), str(src), "-o",
+                           str(exe), "-lpthread"])
+    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
