@@ -509,38 +509,6 @@ BrickFn brick_fn(int cz) {
   return &k_cg_brick_f64<BX, 16>;
 }
 
-int brick_cz_class(int cz) { return cz <= 4 ? 4 : cz <= 8 ? 8 : cz <= 16 ? 16 : 32; }
-
-template <int BX>
-size_t brick_smem(int cz) {
-  using S = BrickShape<BX>;
-  const int c = brick_cz_class(cz);
-  const int rows = (c + S::kLanes - 1) / S::kLanes;  // side ring cells per thread
-  return sizeof(double) *
-         (static_cast<size_t>(c + 1) * S::SXY + 3 * kBT + rows * S::kLanes * S::kSide +
-          c * 2 * S::BY) +
-         sizeof(int) * 6 * kBT;
-}
-
-template <int BX>
-void consider(const Dims &g, int sms, BrickPlan *best, bool *found) {
-  using S = BrickShape<BX>;
-  const int nbx = (g.nx + S::BX - 1) / S::BX, nby = (g.ny + S::BY - 1) / S::BY;
-  if (nbx * nby > sms) return;
-  int nbz = sms / (nbx * nby);
-  const int cz = (g.nz + nbz - 1) / nbz;
-  // a 64-wide brick of more than 16 planes does not fit shared memory
-  if (cz > (S::BX == 64 ? 16 : kBrickMaxPlanes)) return;
-  nbz = (g.nz + cz - 1) / cz;
-  // fewest planes per thread first (0.17 us an iteration each above 4 planes;
-  // below, 36 to 144 CTAs measured the same), then fewest CTAs
-  if (*found && (best->cz < cz || (best->cz == cz && best->ctas() <= nbx * nby * nbz))) return;
-  *best = BrickPlan{S::BX, nbx, nby, nbz, cz, brick_smem<BX>(cz),
-                    2 * sizeof(Packet) * static_cast<size_t>(nbx * nby * nbz) *
-                        brick_inbox_packets(S::kSide, (cz + 3) / 4 * 4)};
-  *found = true;
-}
-
 }  // namespace
 
 bool plan_brick(const Dims &g, BrickPlan *plan) {
@@ -548,13 +516,7 @@ bool plan_brick(const Dims &g, BrickPlan *plan) {
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (sms > 160) sms = 160;  // the sums' polls cover 160 CTAs
-  bool found = false;
-  consider<32>(g, sms, plan, &found);
-  consider<16>(g, sms, plan, &found);
-  consider<64>(g, sms, plan, &found);
-  constexpr size_t kStatic = 2048;  // reduction scratch and scalars, rounded up
-  return found && plan->smem_bytes + kStatic <= static_cast<size_t>(smem);
+  return plan_brick_on(g, sms, smem, plan);
 }
 
 namespace {

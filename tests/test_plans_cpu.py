@@ -1,11 +1,16 @@
-"""Which grids beyond the chip take the one-sweep streaming CG (csrc/afl_sweep_plan.h), with
-the CTAs of 148 SMs and an L2 of 126 MiB: those on which it measured faster than two passes,
-and none of those on which mostly empty tiles or idle CTAs made it slower."""
+"""The plans of the Poisson kernels on a chip of 148 SMs, 227 KB of shared memory per CTA and
+126 MiB of L2.  Which grids beyond the chip take the one-sweep streaming CG
+(csrc/afl_sweep_plan.h): those on which it measured faster than two passes, and none of those
+on which mostly empty tiles or idle CTAs made it slower.  Which bricks a grid on the chip gets
+(csrc/afl_brick.cuh): those that the GPU tests name for it."""
 import subprocess
 
 import pytest
 
+from test_gpu_brick_plans import BRICKS, COLUMNS, SWEEPS
+
 CODE = r"""
+#include "afl_brick.cuh"
 #include "afl_sweep_plan.h"
 #include <cstdio>
 #include <cstdlib>
@@ -15,6 +20,12 @@ int main(int argc, char **v) {
     Dims g{};
     g.nx = atoi(v[q]), g.ny = atoi(v[q + 1]), g.nz = atoi(v[q + 2]);
     g.nxy = g.nx * g.ny, g.n = g.nxy * g.nz;
+    if (atoi(v[q + 3]) == 2) {
+      BrickPlan p{};
+      if (plan_brick_on(g, 148, 227 << 10, &p)) printf("%d,%d,%d\n", p.bx, p.cz, p.ctas());
+      else puts("none");
+      continue;
+    }
     const bool f64 = atoi(v[q + 3]) == 0;
     const int nc = sweep_wide(g) || !f64 ? 4 : 1, ctas = f64 && nc == 4 ? 148 : 296;
     const SweepPlan pl = sweep_plan(g, nc, ctas);
@@ -53,13 +64,15 @@ def plans(tmp_path_factory):
     src, exe = d / "t.cu", d / "t"
     src.write_text(CODE)
     subprocess.check_call([build.nvcc(), *build.ARCH, "-std=c++17", "-O1",
-                           "--expt-relaxed-constexpr", "-I", build.CSRC, str(src), "-o", str(exe)])
+                           "--expt-relaxed-constexpr", "-extended-lambda", "-I", build.CSRC,
+                           str(src), "-o", str(exe)])
 
     def run(shapes, precision):
         args = [str(x) for s in shapes for x in (*s, precision)]
         out = subprocess.run([str(exe), *args], capture_output=True, text=True, timeout=60)
         assert out.returncode == 0, out.stdout
-        return dict(zip(shapes, (w == "1" for w in out.stdout.split())))
+        words = out.stdout.split()
+        return dict(zip(shapes, words if precision == 2 else (w == "1" for w in words)))
     return run
 
 
@@ -73,3 +86,17 @@ def test_sweep_where_it_is_faster(plans, precision):
 def test_two_passes_where_the_sweep_is_slower(plans, precision):
     got = plans(SLOWER[precision], precision)
     assert not any(got.values()), got
+
+
+def test_brick_plans_of_the_gpu_tests(plans):
+    assert plans(list(BRICKS), 2) == {s: "%d,%d,%d" % p for s, p in BRICKS.items()}
+    assert set(plans(list(COLUMNS), 2).values()) == {"none"}
+    reached = {(bx, next(c for c in (4, 8, 16, 32) if cz <= c)) for bx, cz, _ in BRICKS.values()}
+    assert reached >= {(bx, c) for bx in (16, 64) for c in (4, 8, 16, 32) if (bx, c) != (64, 32)}
+    assert any(ctas == 148 for _, _, ctas in BRICKS.values())
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_sweeps_of_the_gpu_tests(plans, precision):
+    got = plans([s for s, p in SWEEPS if p == precision], precision)
+    assert got and all(got.values()), got
