@@ -145,6 +145,10 @@ __global__ void __launch_bounds__(kBT, 1) k_sor_brick(const __grid_constant__ Br
         P[fc.side_d + n * S::kLanes * SXY] = a.p[(k * g.ny + fc.sj) * g.nx + fc.si];
     }
   }
+  // What was read of the neighbours' pressure stays ordered before their writes of it at
+  // the end: they have had a packet of this CTA's by then, and the fence there is the
+  // other half.
+  __threadfence();
   __syncthreads();
 
   const T omega = T(a.omega), keep = T(1) - omega;
@@ -268,6 +272,8 @@ __global__ void __launch_bounds__(kBT, 1) k_sor_brick(const __grid_constant__ Br
       if (!__syncthreads_and(ok)) return;
     }
   }
+  __threadfence();
+  __syncthreads();
 #pragma unroll
   for (int m = 0; m < CZ; ++m) {
     const int k = k0 + m;
