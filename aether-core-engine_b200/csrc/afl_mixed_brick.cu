@@ -362,8 +362,10 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
     ++tag;
     outer_residual();
     brick_partials(acc, red);
-    brick_publish<false>(bs, tag, red);
+    // what it read of the neighbours' pressure comes before the next pass's writes
+    brick_publish<true>(bs, tag, red);
     if (!brick_gather(bs, tag, tot, red + 4 * kBW, true)) return;
+    __threadfence();
     ++tag;
     rr = tot[0];
     ++passes;
