@@ -181,9 +181,10 @@ __device__ __forceinline__ void brick_publish(const Sums &bs, unsigned tag, cons
   }
 }
 
-// The fixed-order total of sum number `tag` in every thread: thread t polls value t & 3 of CTA t / 4 (and of CTA t / 4 + 128), warps and
-// then the CTA add them up.  `ok` (this thread's waits so far) is combined over
-// the CTA; false = a wait gave up and the kernel must unwind.
+// The fixed-order total of sum number `tag` in every thread: thread t polls value t & 3
+// of CTA t / 4 (and of CTA t / 4 + 128), warps and then the CTA add them up.  `ok`
+// (this thread's waits so far) is combined over the CTA; false = a wait gave up and
+// the kernel must unwind.
 __device__ __forceinline__ bool brick_gather(const BrickSums &bs, unsigned tag, double (&out)[4],
                                              double *red, bool ok) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -493,15 +494,16 @@ __device__ __forceinline__ void run_queue(const BrickQueue<Args> &q, Args &a, Qu
 }
 
 // ---- tensor memory as per-thread storage -------------------------------------------
-// Every load, store and wait below starts with __syncwarp(): the .sync.aligned
-// forms need the whole warp converged, and a branch that only some lanes took
-// just before does not promise that (an illegal instruction otherwise).
+// Everything below starts with __syncwarp(): the .sync.aligned forms need the whole
+// warp converged, and a branch that only some lanes took just before does not
+// promise that (an illegal instruction otherwise).
 // 128 lanes x 512 columns of 32 bits beside the register file and shared
 // memory.  Warp w reaches lanes 32*(w%4) .. +31 and owns a quarter of the
 // allocated columns; 32x32b loads and stores move a thread's own columns.
 template <int COLS>
 __device__ __forceinline__ void brick_tm_alloc(unsigned *dst_smem) {  // one whole warp
   const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(dst_smem));
+  __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa),
                "n"(COLS)
                : "memory");
@@ -509,6 +511,7 @@ __device__ __forceinline__ void brick_tm_alloc(unsigned *dst_smem) {  // one who
 }
 template <int COLS>
 __device__ __forceinline__ void brick_tm_dealloc(unsigned taddr) {  // the allocating warp
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(COLS)
                : "memory");
 }

@@ -24,8 +24,10 @@
 //   36 x 52 x 36 7.6 -> 3.1 us.
 // What mattered, in this order: q and p in tensor memory and r in registers (no
 // vector in L2); all packet loads of a thread in flight at once (one after the
-// other: +3 us at 128^3); nothing spilled (the shared-memory carve-out leaves no
-// L1 for local memory: +4 us); packets polled before the sum (+0.8 us after it).
+// other: +3 us at 128^3); no vector spilled (the shared-memory carve-out leaves no
+// L1 for local memory: +4 us; the instances of 32 planes still spill 108 bytes of
+// addresses and scalars a thread, 180 in the queue); packets polled before the sum
+// (+0.8 us after it).
 // Tried and slower: polling the neighbours' sum slots before asking for their
 // packets, and pushing the partial sums into a mailbox per reader (+2 us: the
 // extra words crowd the lines being waited for).

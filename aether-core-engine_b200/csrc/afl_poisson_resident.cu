@@ -404,12 +404,14 @@ constexpr unsigned kTmCols = 512;
 
 __device__ __forceinline__ void tm_alloc_all(unsigned *dst_smem) {  // one whole warp
   const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(dst_smem));
+  __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa),
                "r"(kTmCols)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tm_dealloc_all(unsigned taddr) {  // the allocating warp
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr),
                "r"(kTmCols)
                : "memory");

@@ -255,19 +255,16 @@ NCU_TRAFFIC = {("k_cg_brick_f64", 128): 33.69e6 + 0.41e6,
                ("k_cg_brick_mixed", 128): 34.29e6 + 0.35e6}
 
 
-def poisson_kernel(form, n, resident):
-    """The kernel that solves the pressure of an n^3 grid (afl_cg_sweep.cu has the rule for
-    the grids beyond the chip)."""
+def poisson_kernel(form, resident):
+    """The kernel that solves the pressure of a cubic grid; beyond the chip the library takes one
+    of two by its own rule (afl_sweep_plan.h)."""
     f64 = form.startswith("fp64")
     kind = "f64" if f64 else "mixed"
     if form.endswith("sor"):
         return "k_sor_brick" if resident else "k_rbsor_" + kind
     if resident:
         return "k_cg_brick_" + kind
-    full_tiles = (n + 127) // 128 * 128 <= 1.27 * n
-    sweep = (n % 2 == 0 and 40 * n ** 3 > 126 << 20) if f64 else \
-        (n % 4 == 0 and 16 * n ** 3 > 126 << 20 and full_tiles)
-    return ("k_cg_sweep_" if sweep else "k_cg_stream_") + kind
+    return f"k_cg_sweep_{kind} or k_cg_stream_{kind}"
 
 
 def measured_peak():
@@ -706,7 +703,7 @@ def run_ours(args):
         pois_ms, pois_calls = head["stages"]["poisson"]
         pois_bytes = poisson_bytes(cells, headline, head["infos"])
         achieved = pois_bytes / pois_calls / (pois_ms / pois_calls / 1e3) / 1e9
-        pois_kernel = poisson_kernel(headline, args.n, head["plan"]["resident"])
+        pois_kernel = poisson_kernel(headline, head["plan"]["resident"])
         variants = {}
         for form, r in results.items():
             its = [i.iterations for i in r["infos"]]
