@@ -227,11 +227,16 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
             for (int e = 0; e < 4; ++e) X[(4 * ch + e) * XSTEP + xstage] = q[4 * ch + e];
           }
           if (fc.ydst >= 0) {
+            if (!Sums::kQueued || 4 * ch + 4 <= cl.nzb) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (const int at = S::template y_at<Sums::kQueued>(fc.ydst, 4 * ch + e, cl.nzb);
-                  at >= 0)
-                st_packet(box + at, q[4 * ch + e], tag);
+              for (int e = 0; e < 4; ++e)
+                st_packet(box + S::y_at(fc.ydst, 4 * ch + e, 4 * ch + 4), q[4 * ch + e], tag);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (const int at = S::y_at(fc.ydst, 4 * ch + e, cl.nzb); at >= 0)
+                  st_packet(box + at, q[4 * ch + e], tag);
+            }
           }
           if (ch == 0 && fc.zlo_dst >= 0) st_packet(box + fc.zlo_dst, q[0], tag);
           if (4 * ch + 4 >= cz && fc.zhi_dst >= 0) {

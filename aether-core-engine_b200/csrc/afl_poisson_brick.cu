@@ -265,10 +265,16 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Su
             for (int e = 0; e < 4; ++e) X[(4 * ch + e) * XSTEP + xstage] = qv[e];
           }
           if (ydst >= 0) {
+            if (!Sums::kQueued || 4 * ch + 4 <= cl.nzb) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (const int at = S::template y_at<Sums::kQueued>(ydst, 4 * ch + e, cl.nzb); at >= 0)
-                st_packet(box + at, qv[e], tag);
+              for (int e = 0; e < 4; ++e)
+                st_packet(box + S::y_at(ydst, 4 * ch + e, 4 * ch + 4), qv[e], tag);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (const int at = S::y_at(ydst, 4 * ch + e, cl.nzb); at >= 0)
+                  st_packet(box + at, qv[e], tag);
+            }
           }
           if (ch == 0) {
             const int zlo = I[kZlo];

@@ -34,7 +34,7 @@ int check(int nx, int ny, int nz, int cz) {
           if (at >= 0 && !sent.insert(at).second) printf("sent twice\n"), exit(1);
         };
         for (int m = 0; m < CZ && m < (cz + 3) / 4 * 4; ++m)
-          send(S::template y_at<true>(fc.ydst, m, cl.nzb));
+          send(S::y_at(fc.ydst, m, cl.nzb));
         for (int n = 0; n < CZ / S::kXLanes || n == 0; ++n)
           send(S::template x_at<true>(fc.xdst, t, n, cz, cl.nzb));
         send(fc.zlo_dst);
