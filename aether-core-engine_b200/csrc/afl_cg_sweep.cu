@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kBT, NC == 4 ? 1 : 2)
       for (int c = t0; c < g.n; c += stride) p[c] = __fma_rn(alpha, d[c], p[c]);
     }
   }
-  if (walls != 0.0) {
+  if (it > 0 && walls != 0.0) {  // without a step 0 * inf would be added
     for (int c = t0; c < g.n; c += stride) {
       const Run ru = decode_run<1>(g, c);
       if (!interior(g, ru.i0, ru.j, ru.k)) p[c] += gain * a.b[c];

@@ -422,7 +422,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Su
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t2));  // kept apart: no register across the loop
   const BrickCells<S> cw(g, a.nbx, a.nby, cz, t2, bs.block());
   __syncthreads();
-  const bool wall = keep[3] != 0.0;
+  const bool wall = it > 0 && keep[3] != 0.0;  // without a step 0 * inf would be added
   const double gain = keep[5];
 #pragma unroll
   for (int ch = 0; ch < NCH; ++ch) {

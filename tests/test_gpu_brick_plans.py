@@ -92,6 +92,25 @@ def test_ragged_sweep_matches_numpy(af, shape, precision, iters):
     assert abs(info.final_residual - res) <= (1e-3 if precision else 1e-9) * res
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", [(40, 20, 18), (205, 168, 37), (160, 160, 161)],
+                         ids=["bricks", "columns", "sweep"])
+def test_pressure_untouched_by_a_nan_on_a_wall(af, shape, precision):
+    """A right-hand side that is NaN, or infinite with no iterations to do, on a wall cell
+    stops the solve before its first step: the pressure stays as it was, the NaN is reported."""
+    b, p0 = system(shape, 23, False)
+    for bad, iters in ((np.nan, 5), (np.inf, 0)):
+        if precision and iters == 0:
+            continue  # the mixed form does one iteration at least
+        s = af.FluidSolver3D(*shape, precision=precision, mixed_max_refinements=1)
+        s.set_field("divergence", np.concatenate(([bad], b[1:])))
+        s.set_field("pressure", p0)
+        with pytest.raises(af.AetherFluidError):
+            s.solve_poisson_conjugate_gradient(iters)
+        assert np.array_equal(s.get_field("pressure"), p0)
+        s.close()
+
+
 # every kernel with waits of its own: its shape, precision and solver
 WAITS = {"mixed bricks": ((64, 64, 64), 1, "conjugate_gradient"),
          "sor bricks": ((64, 64, 64), 0, "gauss_seidel"),
