@@ -247,10 +247,10 @@ struct Cells {
 // The reference operator (src/fluid.rs:356-394) on the thread's column of
 // CPT cells, marching up in z with the z neighbours in registers.  No
 // branches or selects: a neighbour the reference skips is a cell outside the
-// interior, where the direction is exactly 0 (r = b - A p = 0 on every
+// interior, where the direction is exactly 0 (r starts at 0 on every
 // non-interior cell, and d = r + beta*d keeps it 0), so adding it leaves the
-// neighbour sum's value unchanged; the sum keeps the reference's order
-// (x-, x+, y-, y+, z-, z+).  The diagonal is the count of interior
+// neighbour sum's value unchanged (a right-hand side on the walls is kept out of r
+// and d: cg_f64_body); the sum keeps the reference's order (x-, x+, y-, y+, z-, z+).  The diagonal is the count of interior
 // neighbours.  Only interior cells keep the result; their neighbours all lie
 // in the grid, so slots that hold no grid cell (halo outside the grid,
 // padding planes) never reach a kept result.
@@ -470,12 +470,17 @@ __device__ __forceinline__ void tm_st4(unsigned taddr, const double (&v)[4]) {
 //    owner's expression, bit for bit.  The pairs are kept by iteration parity.
 //  * The stencil marches up each thread's column with the z neighbours in
 //    registers and no selects (d is exactly 0 off the interior).
+//  * A d is 0 on wall cells and interior cells skip them, so their r stays b, their
+//    d = s_k b with s_0 = 1, s_{k+1} = 1 + beta_k s_k, and p gains b times the sum of
+//    alpha_k s_k.  They are left out of r and d: their r.r joins the sums as one
+//    number (wall[0]), and p gets its gain at the end (b is 0 there after a
+//    divergence; a caller's own right-hand side may not be).
 // The arguments are __grid_constant__: they stay in the constant bank.
 template <int TY, int CPT>
 __device__ __forceinline__ void cg_f64_body(const ResidentCgArgs &a, const GridSync &gs,
                                             const TagSync &ts, double *D, double *scratch,
-                                            double *slot, double *vals, unsigned t_r,
-                                            unsigned t_p) {
+                                            double *slot, double *vals, double *wall,
+                                            unsigned t_r, unsigned t_p) {
   using C = Cells<TY, CPT>;
   constexpr int NCH = (CPT + 3) / 4;  // chunks of 4 doubles in TMEM
   const Dims g = a.g;
@@ -491,7 +496,7 @@ __device__ __forceinline__ void cg_f64_body(const ResidentCgArgs &a, const GridS
   {
     // r = b - A p (src/fluid.rs:455-458) and p into TMEM, d = r.  The chunk
     // loops stay rolled: unrolled over 16 cells they spill.
-    double acc[2] = {0.0, 0.0};
+    double acc[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
     for (int ch = 0; ch < NCH; ++ch) {
       double rv4[4] = {0.0, 0.0, 0.0, 0.0}, pv4[4] = {0.0, 0.0, 0.0, 0.0};
@@ -501,25 +506,32 @@ __device__ __forceinline__ void cg_f64_body(const ResidentCgArgs &a, const GridS
         if (m >= CPT) break;
         if (cl.valid(g, m)) {
           const int c = cl.c0 + m * g.nxy;
-          const double ap = cl.interior(g, m) ? lap_global(g, p, c, cl.i, cl.j, cl.k0 + m) : 0.0;
+          const bool in = cl.interior(g, m);
+          const double ap = in ? lap_global(g, p, c, cl.i, cl.j, cl.k0 + m) : 0.0;
           const double bc = __ldg(a.b + c);
           const double rv = bc - ap;
-          rv4[q] = rv;
+          rv4[q] = in ? rv : 0.0;
           pv4[q] = __ldcg(p + c);
-          if (cl.edge) pr0[c].x = rv;
+          if (cl.edge) pr0[c].x = rv4[q];
           acc[0] += rv * rv;
           acc[1] += bc * bc;
+          acc[2] += in ? 0.0 : bc * bc;
         }
         D[cl.s0 + m * C::SXY] = rv4[q];
       }
       tm_st4(t_r + 8u * ch, rv4);
       tm_st4(t_p + 8u * ch, pv4);
     }
-    tag_publish<2>(ts, unsigned(phase + 1), acc, scratch);
+    tag_publish<3>(ts, unsigned(phase + 1), acc, scratch);
   }
-  double tot[2];
-  if (!tag_gather<2>(ts, gs, unsigned(phase + 1), tot, slot, vals)) return;
+  double tot[3];
+  if (!tag_gather<3>(ts, gs, unsigned(phase + 1), tot, slot, vals)) return;
   ++phase;
+  if (threadIdx.x == 0) {
+    wall[0] = tot[2];
+    wall[1] = 1.0;  // s_k
+    wall[2] = 0.0;  // the sum of alpha_k s_k
+  }
   double delta = tot[0];
   const double bb = tot[1];
   double tol2 = -1.0;
@@ -594,6 +606,11 @@ __device__ __forceinline__ void cg_f64_body(const ResidentCgArgs &a, const GridS
       const double beta = dnext / delta;
       // p += alpha d, r -= alpha q, d = r + beta d (src/fluid.rs:472-485)
       rr_next = 0.0;
+      if (threadIdx.x == 0) {
+        wall[2] += alpha * wall[1];
+        wall[1] = 1.0 + beta * wall[1];
+        if (blockIdx.x == 0) rr_next = wall[0];
+      }
       // r and q of a chunk come from this thread's published pairs in L2 (r
       // as in TMEM, bit for bit); the next chunk's loads are issued after this
       // chunk's TMEM stores, when its registers are free, so their latency
@@ -641,6 +658,8 @@ __device__ __forceinline__ void cg_f64_body(const ResidentCgArgs &a, const GridS
     }
   }
   // the pressure back to global memory
+  __syncthreads();
+  const bool gains = it > 0 && wall[0] != 0.0;  // without a step 0 * inf would be added
 #pragma unroll 1
   for (int ch = 0; ch < NCH; ++ch) {
     double pv4[4];
@@ -648,7 +667,11 @@ __device__ __forceinline__ void cg_f64_body(const ResidentCgArgs &a, const GridS
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int m = ch * 4 + q;
-      if (m < CPT && cl.valid(g, m)) p[cl.c0 + m * g.nxy] = pv4[q];
+      if (m < CPT && cl.valid(g, m)) {
+        const int c = cl.c0 + m * g.nxy;
+        if (gains && !cl.interior(g, m)) pv4[q] += wall[2] * __ldg(a.b + c);
+        p[c] = pv4[q];
+      }
     }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && a.report) {
@@ -672,14 +695,15 @@ __global__ void __launch_bounds__(kRT, 1)
   extern __shared__ double Dbase[];
   __shared__ double scratch[kScratch];
   __shared__ double vals[kMaxTagBlocks * kMaxNV];
+  __shared__ double wall[3];
   __shared__ unsigned tm_base;
   const int warp = threadIdx.x >> 5;
   if (warp == 0) tm_alloc_all(&tm_base);
   tm_sync_threads();
   // this thread's 64 columns: r in the first 32, p in the next 32
   const unsigned t_r = tm_base + ((32u * unsigned(warp & 3)) << 16) + 64u * unsigned(warp >> 2);
-  cg_f64_body<TY, CPT>(a, gs, ts, Dbase + C::SXY, scratch, scratch + kScratchSlot, vals, t_r,
-                       t_r + 32u);
+  cg_f64_body<TY, CPT>(a, gs, ts, Dbase + C::SXY, scratch, scratch + kScratchSlot, vals, wall,
+                       t_r, t_r + 32u);
   tm_sync_threads();  // every TMEM access of the CTA is complete
   if (warp == 0) tm_dealloc_all(tm_base);
 }
@@ -698,6 +722,7 @@ __global__ void __launch_bounds__(kRT, 1)
   float *Df = Dfbase + C::SXY;  // one padding plane below plane 0
   __shared__ double scratch[kScratch];
   __shared__ double vals[kMaxTagBlocks * kMaxNV];
+  __shared__ double wall[3];  // of the wall cells, as in the FP64 kernel: r.r, s_k, their gain
   double *slot = scratch + kScratchSlot;
   const Dims g = a.g;
   const C cl(g, a.tiles_x);
@@ -710,31 +735,34 @@ __global__ void __launch_bounds__(kRT, 1)
 
   // r = b - A p in f64, rounded once to f32; e = 0.
   auto outer_residual = [&](bool with_b) {
-    double acc[3] = {0.0, 0.0, 0.0};
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int m = 0; m < CPT; ++m) {
       r[m] = 0.0f;
       e[m] = 0.0f;
       if (!cl.valid(g, m)) continue;
       const int c = cl.c0 + m * g.nxy;
-      const double ap = cl.interior(g, m) ? lap_global(g, p, c, cl.i, cl.j, cl.k0 + m) : 0.0;
+      const bool in = cl.interior(g, m);
+      const double ap = in ? lap_global(g, p, c, cl.i, cl.j, cl.k0 + m) : 0.0;
       const double bc = __ldg(a.b + c);
       const double rv = bc - ap;
       const float rf = float(rv);
-      r[m] = rf;
-      if (cl.edge) rpub[c] = rf;
+      r[m] = in ? rf : 0.0f;
+      if (cl.edge) rpub[c] = r[m];
       acc[0] += rv * rv;
       if (with_b) acc[1] += bc * bc;
       acc[2] += double(rf) * double(rf);
+      acc[3] += in ? 0.0 : double(rf) * double(rf);
     }
-    tag_publish<3>(ts, unsigned(phase + 1), acc, scratch);
+    tag_publish<4>(ts, unsigned(phase + 1), acc, scratch);
   };
 
   outer_residual(true);
-  double tot[3];
-  if (!tag_gather<3>(ts, gs, unsigned(phase + 1), tot, slot, vals)) return;
+  double tot[4];
+  if (!tag_gather<4>(ts, gs, unsigned(phase + 1), tot, slot, vals)) return;
   ++phase;
   const double bb = tot[1];
+  if (threadIdx.x == 0) wall[0] = tot[3];
   double rr = tot[0];
   const double rr0 = rr;
   double tol2 = -1.0;
@@ -751,6 +779,10 @@ __global__ void __launch_bounds__(kRT, 1)
     double delta = tot[2];
     const double inner_tol2 = inner_rel * inner_rel * delta;
     double beta = 0.0;
+    if (threadIdx.x == 0) {
+      wall[1] = 1.0;
+      wall[2] = 0.0;
+    }
     int it = 0;
     while (it < a.max_inner && total < a.max_iters) {
       const bool first = it == 0;
@@ -778,6 +810,9 @@ __global__ void __launch_bounds__(kRT, 1)
       if (!(fabs(dq[0]) >= 1e-30)) break;
       const float af = float(delta / dq[0]);
       double acc2[1] = {0.0};
+      if (threadIdx.x == 0) {
+        wall[2] += double(af) * wall[1];
+      }
 #pragma unroll
       for (int m = 0; m < CPT; ++m) {
         const int s = cl.s0 + m * C::SXY;
@@ -788,6 +823,7 @@ __global__ void __launch_bounds__(kRT, 1)
         if (cl.edge && cl.valid(g, m)) rpub[cl.c0 + m * g.nxy] = rv;
         acc2[0] += double(rv) * double(rv);
       }
+      if (blockIdx.x == 0 && threadIdx.x == 0) acc2[0] += wall[0];
       tag_publish<1>(ts, unsigned(phase + 1), acc2, scratch);
       double dn[1];
       if (!tag_gather<1>(ts, gs, unsigned(phase + 1), dn, slot, vals)) return;
@@ -797,17 +833,21 @@ __global__ void __launch_bounds__(kRT, 1)
       if (!isfinite(dn[0]) || dn[0] <= inner_tol2 || dn[0] < 1e-30) break;
       beta = dn[0] / delta;
       delta = dn[0];
+      if (threadIdx.x == 0) wall[1] = 1.0 + double(float(beta)) * wall[1];
     }
     // p += e in f64, then the true residual again.
+    __syncthreads();
+    const bool gains = wall[0] != 0.0;
 #pragma unroll
     for (int m = 0; m < CPT; ++m) {
       if (!cl.valid(g, m)) continue;
       const int c = cl.c0 + m * g.nxy;
+      if (gains && !cl.interior(g, m)) e[m] = float(__ldg(a.b + c) * wall[2]);
       p[c] = p[c] + double(e[m]);
     }
     if (!grid_sync(gs)) return;
     outer_residual(false);
-    if (!tag_gather<3>(ts, gs, unsigned(phase + 1), tot, slot, vals)) return;
+    if (!tag_gather<4>(ts, gs, unsigned(phase + 1), tot, slot, vals)) return;
     ++phase;
     rr = tot[0];
     ++passes;

@@ -93,6 +93,26 @@ def test_ragged_sweep_matches_numpy(af, shape, precision, iters):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("shape", [(64, 64, 75), *COLUMNS, (160, 160, 161)],
+                         ids=["bricks", "columns16", "columns8", "columns4", "sweep"])
+def test_right_hand_side_on_the_walls_matches_oracle(af, oracle, shape, precision):
+    """Three iterations on a right-hand side of the caller's own that is not 0 on two walls,
+    which the operator neither reads nor changes."""
+    nx, ny, nz = shape
+    b, p0 = system(shape, 25, False)
+    b = b.reshape(nz, ny, nx)
+    b[0], b[:, :, -1] = 0.01, -0.02
+    o = oracle.OracleSolver(*shape)
+    o.field("divergence")[:] = b.ravel()
+    o.field("pressure")[:] = p0
+    assert o.solve_poisson_conjugate_gradient(3) == 3
+    got, info = solve(af, shape, 0, b.ravel(), p0, 3, precision=precision,
+                      mixed_max_refinements=1)
+    assert info.iterations == 3
+    assert rel_l2(got, np.array(o.field("pressure"))) <= (1e-4 if precision else 1e-10)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("shape", [(40, 20, 18), (205, 168, 37), (160, 160, 161)],
                          ids=["bricks", "columns", "sweep"])
 def test_pressure_untouched_by_a_nan_on_a_wall(af, shape, precision):
