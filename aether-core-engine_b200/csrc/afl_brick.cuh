@@ -227,8 +227,9 @@ struct BrickShape {
   // thread's n-th side ring cell is waited for.  In a queue a CTA sends exactly what is
   // waited for: a packet that nobody reads could land after its receiver has gone on to
   // another system and cleared its inbox for that one.  A launch with one system has no
-  // such next one, and sends its last chunk's padding planes as well: tests of every plane
-  // cost it 3 % of an iteration of 128^3 (mixed 9 %).  A queue tests a whole chunk first
+  // such next one, and sends its last chunk's padding planes and the rows past the grid as
+  // well: tests of every plane cost it 3 % of an iteration of 128^3 (mixed 9 %), the test of
+  // the rows alone 2 % of mixed 36 x 52 x 36.  A queue tests a whole chunk first
   // (the 48 plumes, 4 steps, tests of every plane -> this: 46.5 -> 45.4 ms).
   static __host__ __device__ __forceinline__ int y_at(int ydst, int m, int nzb) {
     return ydst >= 0 && m < nzb ? ydst + m * kSide : -1;
@@ -286,7 +287,8 @@ struct BrickCells {
 // and the last lane of a row hold, are staged in shared memory ([plane][x-
 // rows, x+ rows]) and sent by all threads: thread t sends staged row
 // t % (2 * BY) of every kXLanes-th plane.
-template <typename S>
+// QUEUED: rows past the grid have no x face (BrickShape::x_at).
+template <typename S, bool QUEUED = false>
 struct BrickFaces {
   int xstage;         // this column's staged row (-1: not on an x face)
   int xdst;           // where the thread's first staged value goes; kSide packets per plane
@@ -312,7 +314,7 @@ struct BrickFaces {
       const int xs = t % (2 * S::BY), m0 = t / (2 * S::BY) * S::kSide;
       xdst = xs < S::BY ? (cl.bx > 0 ? box(-1, 0, 0) + S::BY + xs + m0 : -1)
                         : (cl.bx + 1 < nbx ? box(1, 0, 0) + xs - S::BY + m0 : -1);
-      if (cl.by * S::BY + xs % S::BY >= g.ny) xdst = -1;  // a row past the grid
+      if (QUEUED && cl.by * S::BY + xs % S::BY >= g.ny) xdst = -1;
     }
     xcol = -1;
     if (cl.in_ij) {

@@ -62,7 +62,7 @@ __device__ __forceinline__ void cg_brick_mixed_body(const BrickMixedArgs &a, con
   const int t = threadIdx.x;
   const int cz = a.cz;
   const BrickCells<S> cl(g, a.nbx, a.nby, cz, t, bs.block());
-  const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp, t);
+  const BrickFaces<S, Sums::kQueued> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp, t);
   const int k0 = cl.z0, k_lo = 2 - k0, k_hi = min(g.nz - 3 - k0, cl.nzb - 1);
   const bool col_in = cl.column_interior(g);
   const bool side_in = fc.si >= 1 && fc.si <= g.nx - 2 && fc.sj >= 1 && fc.sj <= g.ny - 2;

@@ -96,7 +96,7 @@ __device__ __forceinline__ void cg_brick_f64_body(const BrickCgArgs &a, const Su
   const int t = threadIdx.x;
   const int cz = a.cz;
   const BrickCells<S> cl(g, a.nbx, a.nby, cz, t, bs.block());
-  const BrickFaces<S> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp, t);
+  const BrickFaces<S, Sums::kQueued> fc(g, cl, a.nbx, a.nby, a.nbz, a.czp, t);
   // z of the brick's plane m is k0 + m; chunks whose four planes all have both
   // z neighbours take the plain path of the operator
   const int k0 = cl.z0, k_lo = 2 - k0, k_hi = min(g.nz - 3 - k0, cl.nzb - 1);

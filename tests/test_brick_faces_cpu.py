@@ -29,7 +29,7 @@ int check(int nx, int ny, int nz, int cz) {
     for (int b = 0; b < nbx * nby * nbz; ++b)
       for (int t = 0; t < kBT; ++t) {
         const BrickCells<S> cl(g, nbx, nby, cz, t, b);
-        const BrickFaces<S> fc(g, cl, nbx, nby, nbz, czp, t);
+        const BrickFaces<S, true> fc(g, cl, nbx, nby, nbz, czp, t);
         auto send = [&](int at) {
           if (at >= 0 && !sent.insert(at).second) printf("sent twice\n"), exit(1);
         };
