@@ -27,7 +27,7 @@
 // into L2.  Measured with streaming solves on the 48-plume ensemble (mixed, 100 steps,
 // autotuned): 645-650 Mcell-steps/s against 632-633 for the graph of stage launches (593
 // without the prefetch), so this became the default form.  With solves on chip the order
-// is the other way round, 975-979 against 1023-1024; the default stays, because the f32
+// is the other way round, 957-979 against 1002-1024; the default stays, because the f32
 // stages of the two forms round differently and a caller's results would change with it.
 #define AFL_RESTRICT
 #include <type_traits>

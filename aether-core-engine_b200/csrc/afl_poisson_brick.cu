@@ -568,7 +568,7 @@ int launch_cg_brick(const BrickSolve &s, const BrickPlan &plan, cudaStream_t st)
 //
 // Against the streaming solve, which takes every system at once at 6.6 ps a cell and
 // iteration (FP64 13) and not less than 4 us an iteration.  ms per step, streaming -> this:
-// the 48 plumes 16.2 -> 11.3 (FP64 31.4 -> 11.9), one 32^3 1.6 -> 0.44, one 128^3 5.2 -> 2.4,
+// the 48 plumes 16.2 -> 11.4 (FP64 31.4 -> 11.9), one 32^3 1.6 -> 0.44, one 128^3 5.2 -> 2.4,
 // 140 of 16^3 1.6 -> 0.9, 9 of 96^3 13.2 -> 11.0; several per CTA on bricks that the grids
 // leave half empty lose in f32: 40 of 40^3 3.8 -> 4.5 (FP64 5.2 -> 4.5), 300 of 16^3
 // 2.0 -> 2.2 (2.5 -> 2.2).

@@ -312,8 +312,9 @@ afl_status afl_ensemble_tile_depth(const afl_ensemble *e, int32_t *kz);
  * instance meeting at the instance's own bounded barrier between stages
  * (the default when the step kernel's co-resident CTAs outnumber the
  * instances); 0 = the captured graph of per-stage batched launches plus the
- * cooperative solve, 4-5 % faster on 48 plumes whose solves run on chip.  Setting it re-splits the CTAs for the form's
- * co-resident budget, clears the autotune choice and captures the step again. */
+ * cooperative solve, 4-5 % faster on 48 plumes whose solves run on chip.
+ * Setting it re-splits the CTAs for the form's co-resident budget, clears the
+ * autotune choice and captures the step again. */
 afl_status afl_ensemble_set_persistent(afl_ensemble *e, int32_t on);
 afl_status afl_ensemble_persistent(const afl_ensemble *e, int32_t *on);
 /* The reference generator (src/rng.rs:21-88): n values of next_f64 after
